@@ -39,6 +39,23 @@ __device__ __forceinline__ uint64_t xorshift_jump(const uint64_t* __restrict__ n
   return state;
 }
 
+// xorshift_jump by a count that is the same for the whole warp, all 32 lanes
+// calling together: lane q looks up nibble q and two warp reductions combine
+// the 16 images, about 12 instructions per set bit instead of about 100.
+__device__ __forceinline__ uint64_t xorshift_jump_uniform(const uint64_t* __restrict__ nibble, uint64_t state,
+                                                          uint64_t k) {
+  const uint32_t lane = threadIdx.x & 31u, q = lane & 15u;
+  while (k) {
+    const int b = __ffsll((long long)k) - 1;
+    uint64_t y = __ldg(nibble + (size_t)b * 256 + q * 16 + ((state >> (4 * q)) & 0xF));
+    if (lane >= 16) y = 0;
+    state = ((uint64_t)__reduce_xor_sync(0xFFFFFFFFu, (uint32_t)(y >> 32)) << 32) |
+            __reduce_xor_sync(0xFFFFFFFFu, (uint32_t)y);
+    k &= k - 1;
+  }
+  return state;
+}
+
 // Sequential MonteCarloRng positioned at an arbitrary normal index.
 __device__ __forceinline__ float neg2_log_fast(float u);
 

@@ -12,6 +12,7 @@ namespace mpc {
 struct DeviceTables {
   const uint32_t* sobol;  // [256][8][16] nibble tables
   const uint64_t* jump;   // [64][16][16] xorshift jump nibble tables
+  const uint64_t* lane_jump;  // [16][16][32] (q, v, lane): v << 4q jumped kMertonRun * lane draws; contexts only
 };
 
 // Fused FP32 path: one persistent launch over a tile work list.  All
@@ -154,27 +155,31 @@ cudaError_t launch_greeks_single_pass(const GreekArgs& a, uint32_t grid, const D
 
 // The reference's Merton estimator (terminal, pseudorandom): each chunk's
 // sequential MonteCarloRng stream is replayed and the variable number of
-// draws per path resolved by a parallel chain over 64-position segments
-// (mpc_merton.cu).  Per chunk, qpad stream positions (a multiple of
-// kMertonSegment, at least 3 per path plus one spare segment) and n_segs =
-// qpad / kMertonSegment - 1 segments.
-constexpr uint32_t kMertonSegment = 64;
+// draws per path resolved by a parallel chain (mpc_merton.cu).  A block owns
+// kMertonBlockPos stream positions of one chunk; a chunk of n paths takes at
+// most 3 n positions.
+constexpr uint32_t kMertonRun = 16;       // positions per thread
+constexpr uint32_t kMertonThreads = 256;
+constexpr uint32_t kMertonBlockPos = kMertonRun * kMertonThreads;
 struct MertonStreamArgs {
   uint64_t n_paths;             // all chunks
-  uint32_t n_chunks, cv;        // chunk count (1 = one stream); record controls
+  uint32_t n_chunks;            // chunk count (1 = one stream)
+  uint32_t blocks_per_chunk;    // blocks of the launch are chunk-major
   uint64_t chunk_base, chunk_rem;  // the reference's split of n_paths
   uint64_t seed;                // request seed (chunk seeds derived from it)
-  uint64_t qpad, n_segs;
   double mean, p0;              // lambda T and exp(-lambda T)
+  int64_t jump_above;           // a path jumps when its 53-bit uniform exceeds this
   double log_s0, drift_t, vol_t, jump_mean, jump_vol, k, discount;
-  uint64_t* x;                  // [n_chunks][qpad] stream outputs
-  uint32_t* bits;               // [n_chunks][qpad / 32] jump bits
-  uint16_t* maps;               // [n_chunks][n_segs][9] segment maps
-  uint8_t* seg_state;           // [n_chunks][n_segs] entry state
-  unsigned long long* seg_before;  // [n_chunks][n_segs] paths before the segment
-  uint64_t* starts;             // [n_paths] path start states
-  double* payoff;               // [n_paths]
-  double* control;              // [n_paths] or null
+  uint64_t* halo;               // [blocks][4] last stream outputs of a block
+  uint32_t* run_entry;          // [blocks][kMertonThreads] entry class of a run per entry class of its block (nibbles)
+  uint32_t* block_map;          // [blocks][8]: exit state per entry class (nibbles), starts per entry class
+  uint32_t* block_state;        // [blocks] entry state
+  unsigned long long* block_before;  // [blocks] paths of the chunk before the block
+  uint32_t* chunk_done;         // [n_chunks] finished blocks (zero before and after)
+  uint32_t* done;               // finished blocks of the second kernel (zero before and after)
+  double* partials;             // [blocks][2]: sum p, sum p^2
+  double* out;                  // count, sum p, sum p^2
+  double* payoff;               // [n_paths] or null
 };
 cudaError_t launch_merton_stream(const MertonStreamArgs& a, const DeviceTables& tabs, cudaStream_t stream);
 

@@ -90,6 +90,16 @@ int scratch(mpc_context* ctx, const std::string& name, size_t bytes, void** out)
   return MPC_OK;
 }
 
+// Refuses a request whose documented size alone passes the context's budget.
+// The kernels keep less on the device than mpc_estimate_bytes states, but a
+// request beyond the budget stays refused.
+static int within_budget(mpc_context* ctx, const char* name, uint64_t bytes) {
+  if (bytes <= ctx->budget) return MPC_OK;
+  return fail(ctx, MPC_E_OOM_BUDGET,
+              "request needs " + std::to_string(bytes) + " device bytes for '" + name +
+                  "', beyond the HBM budget of " + std::to_string(ctx->budget) + " bytes");
+}
+
 static int pinned_staging(mpc_context* ctx, size_t bytes, void** out) {
   if (ctx->pinned_bytes < bytes) {
     if (ctx->pinned) {
@@ -939,12 +949,12 @@ static int run_plain(mpc_context* ctx, Prepared* p, mpc_result_t* out, double* p
 }
 
 // The reference's terminal pseudorandom Merton: each chunk's MonteCarloRng
-// stream replayed on the device (mpc_merton.cu), payoffs reduced like the
-// plain path.  Both precisions run this FP64 pipeline: its cost is the stream
-// replay, and it reproduces the reference's per-path payoffs.
+// stream replayed on the device (mpc_merton.cu).  Both precisions run this
+// FP64 pipeline: its cost is the stream replay, and it reproduces the
+// reference's per-path payoffs.
 static int run_merton_stream(mpc_context* ctx, Prepared* p, mpc_result_t* out, double* per_unit_host,
                              uint64_t per_unit_cap) {
-  DevReq& q = p->q;
+  const DevReq& q = p->q;
   const uint64_t n = q.n_paths;
   MertonStreamArgs a{};
   a.n_paths = n;
@@ -952,13 +962,11 @@ static int run_merton_stream(mpc_context* ctx, Prepared* p, mpc_result_t* out, d
   a.chunk_base = q.chunk_base;
   a.chunk_rem = q.chunk_rem;
   a.seed = q.seed;
-  a.cv = q.cv;
-  const uint64_t max_chunk = a.n_chunks <= 1 ? n : q.chunk_base + (q.chunk_rem ? 1 : 0);
-  const uint64_t positions = 3 * max_chunk + 8;  // a path reads at most 3 positions past its start
-  a.n_segs = (positions + kMertonSegment - 1) / kMertonSegment;
-  a.qpad = (a.n_segs + 1) * kMertonSegment;  // one spare segment: the last one reads 2 bits past its end
-  a.mean = q.lam_dt;                         // lambda T (terminal: dt = T)
-  a.p0 = q.lam_p0;                           // exp(-lambda T), as sample_poisson computes it
+  a.mean = q.lam_dt;  // lambda T (terminal: dt = T)
+  a.p0 = q.lam_p0;    // exp(-lambda T), as sample_poisson computes it
+  // open01 of the 53-bit uniform m is max(m 2^-53, DBL_MIN); it exceeds p0 exactly when m > floor(p0 2^53),
+  // or always when p0 < DBL_MIN (the scaling is exact)
+  a.jump_above = a.p0 < 2.2250738585072014e-308 ? -1 : int64_t(std::floor(a.p0 * 9007199254740992.0));
   a.log_s0 = q.log_s0;
   a.drift_t = q.drift_dt;
   a.vol_t = q.vol_dt;
@@ -966,57 +974,49 @@ static int run_merton_stream(mpc_context* ctx, Prepared* p, mpc_result_t* out, d
   a.jump_vol = q.jump_vol;
   a.k = q.k;
   a.discount = q.discount;
-  const uint64_t chunks = a.n_chunks, segs = a.n_segs * chunks;
-  void *d_x, *d_bits, *d_maps, *d_state, *d_before, *d_starts = nullptr, *d_pay, *d_ctl = nullptr;
-  void *d_req, *d_part, *d_mom, *d_done;
+  const uint64_t max_chunk = a.n_chunks <= 1 ? n : q.chunk_base + (q.chunk_rem ? 1 : 0);
+  const uint64_t positions = a.mean != 0.0 ? 3 * max_chunk : max_chunk;  // every path starts below this
+  a.blocks_per_chunk = uint32_t((positions + kMertonBlockPos - 1) / kMertonBlockPos);
+  const uint64_t blocks = uint64_t(a.blocks_per_chunk) * a.n_chunks;
+  if (blocks > 0x7FFFFFFFull) return fail(ctx, MPC_E_UNSUPPORTED, "too many stream blocks for one launch");
   int st;
-  if ((st = scratch(ctx, "merton_x", chunks * a.qpad * sizeof(uint64_t), &d_x))) return st;
-  if ((st = scratch(ctx, "merton_bits", chunks * a.qpad / 32 * sizeof(uint32_t), &d_bits))) return st;
-  if ((st = scratch(ctx, "merton_maps", segs * 9 * sizeof(uint16_t), &d_maps))) return st;
-  if ((st = scratch(ctx, "merton_state", segs, &d_state))) return st;
-  if ((st = scratch(ctx, "merton_before", segs * sizeof(uint64_t), &d_before))) return st;
-  if (a.mean != 0.0 && (st = scratch(ctx, "merton_starts", n * sizeof(uint64_t), &d_starts))) return st;
-  if ((st = scratch(ctx, "plain_pay", n * sizeof(double), &d_pay))) return st;
-  if (q.cv && (st = scratch(ctx, "plain_ctl", n * sizeof(double), &d_ctl))) return st;
-  a.x = static_cast<uint64_t*>(d_x);
-  a.bits = static_cast<uint32_t*>(d_bits);
-  a.maps = static_cast<uint16_t*>(d_maps);
-  a.seg_state = static_cast<uint8_t*>(d_state);
-  a.seg_before = static_cast<unsigned long long*>(d_before);
-  a.starts = static_cast<uint64_t*>(d_starts);
+  // the request's documented size counts one 8-byte word per stream position
+  if ((st = within_budget(ctx, "merton stream", a.n_chunks * (3 * max_chunk + 8) * 8))) return st;
+  // run entries | block maps | halo | blocks' path counts | partials | block states
+  const size_t o_map = blocks * kMertonThreads * 4, o_halo = o_map + blocks * 32, o_before = o_halo + blocks * 32,
+               o_part = o_before + blocks * 8, o_state = o_part + blocks * 16, ws_bytes = o_state + blocks * 4;
+  void *d_ws, *d_done, *d_pay = nullptr;
+  if ((st = scratch(ctx, "merton_ws", ws_bytes, &d_ws))) return st;
+  // counters: zero-filled when allocated, and every launch leaves them zero
+  if ((st = scratch(ctx, "merton_done", (size_t(a.n_chunks) + 1) * sizeof(uint32_t), &d_done))) return st;
+  if (per_unit_host && (st = scratch(ctx, "plain_pay", n * sizeof(double), &d_pay))) return st;
+  uint8_t* ws = static_cast<uint8_t*>(d_ws);
+  a.run_entry = reinterpret_cast<uint32_t*>(ws);
+  a.block_map = reinterpret_cast<uint32_t*>(ws + o_map);
+  a.halo = reinterpret_cast<uint64_t*>(ws + o_halo);
+  a.block_before = reinterpret_cast<unsigned long long*>(ws + o_before);
+  a.partials = reinterpret_cast<double*>(ws + o_part);
+  a.block_state = reinterpret_cast<uint32_t*>(ws + o_state);
+  a.done = static_cast<uint32_t*>(d_done);
+  a.chunk_done = a.done + 1;
   a.payoff = static_cast<double*>(d_pay);
-  a.control = static_cast<double*>(d_ctl);
-  q.tile_units = 2048;
-  q.n_tiles = uint32_t((n + q.tile_units - 1) / q.tile_units);
-  if ((st = scratch(ctx, "plain_req", sizeof(DevReq), &d_req))) return st;
-  if ((st = scratch(ctx, "plain_part", size_t(q.n_tiles) * MPC_MOMENTS * sizeof(double), &d_part))) return st;
-  if ((st = scratch(ctx, "plain_mom", MPC_MOMENTS * sizeof(double), &d_mom))) return st;
-  if ((st = scratch(ctx, "plain_done", 16, &d_done))) return st;
-  q.partials = static_cast<double*>(d_part);
-  q.moments = static_cast<double*>(d_mom);
-  q.tiles_done = static_cast<uint32_t*>(d_done);
-  q.per_unit = nullptr;
   void* pin = nullptr;
-  if ((st = pinned_staging(ctx, sizeof(DevReq) + MPC_MOMENTS * sizeof(double), &pin))) return st;
-  std::memcpy(pin, &q, sizeof(DevReq));
-  double* hm = reinterpret_cast<double*>(static_cast<uint8_t*>(pin) + sizeof(DevReq));
+  if ((st = pinned_staging(ctx, MPC_MOMENTS * sizeof(double), &pin))) return st;
+  double* hm = static_cast<double*>(pin);  // written by the kernel itself (pinned memory is mapped)
+  std::memset(hm, 0, MPC_MOMENTS * sizeof(double));
+  a.out = hm;
   uint64_t launches_before = kernel_launch_count();
   MPC_CUDA(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
-  MPC_CUDA(ctx, cudaMemcpyAsync(d_req, pin, sizeof(DevReq), cudaMemcpyHostToDevice, ctx->stream));
-  MPC_CUDA(ctx, cudaMemsetAsync(d_done, 0, 16, ctx->stream));
   cudaError_t e = launch_merton_stream(a, ctx->tabs, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "Merton stream replay");
-  e = launch_plain_reduce(static_cast<DevReq*>(d_req), a.payoff, a.control, n, q.n_tiles, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "Merton reduction");
-  MPC_CUDA(ctx, cudaMemcpyAsync(hm, d_mom, MPC_MOMENTS * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   MPC_CUDA(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
   MPC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
   ctx->last_ms = ms;
   ctx->last_launches = kernel_launch_count() - launches_before;
-  ctx->last_h2d = sizeof(DevReq);
-  ctx->last_d2h = MPC_MOMENTS * sizeof(double);
+  ctx->last_h2d = 0;
+  ctx->last_d2h = 3 * sizeof(double);
   summarize_moments(*p, hm, out);
   out->path_steps = p->path_steps;
   out->runtime_ms = ms;
@@ -1695,6 +1695,24 @@ std::vector<uint64_t> xorshift_jump_table(uint64_t k) {
   return tab;
 }
 
+std::vector<uint64_t> xorshift_lane_table(uint32_t run) {
+  std::vector<uint64_t> tab(16 * 16 * 32, 0ull), cols(64);
+  for (int i = 0; i < 64; ++i) cols[i] = 1ull << i;
+  for (int lane = 0; lane < 32; ++lane) {
+    for (int q = 0; q < 16; ++q)
+      for (int v = 0; v < 16; ++v)
+        for (int j = 0; j < 4; ++j)
+          if ((v >> j) & 1) tab[(q * 16 + v) * 32 + lane] ^= cols[4 * q + j];
+    for (uint64_t& x : cols)
+      for (uint32_t s = 0; s < run; ++s) {
+        x ^= x >> 12;
+        x ^= x << 25;
+        x ^= x >> 27;
+      }
+  }
+  return tab;
+}
+
 void build_tables(std::vector<uint32_t>& sob, std::vector<uint64_t>& jump) {
   sob.assign(size_t(MPC_SOBOL_TABLE_WORDS), 0u);
   build_icdf_segments(&sob[MPC_ICDF_OFFSET]);
@@ -2242,6 +2260,9 @@ int mpc_create(const mpc_options_t* options, mpc_context_t** out) {
   std::vector<uint32_t> sob;
   std::vector<uint64_t> jump;
   build_tables(sob, jump);
+  const size_t lane_at = jump.size();
+  const std::vector<uint64_t> lane_table = xorshift_lane_table(kMertonRun);
+  jump.insert(jump.end(), lane_table.begin(), lane_table.end());
   if ((e = cudaMalloc(&ctx->d_sobol, sob.size() * 4)) != cudaSuccess) return bail(e, "cudaMalloc tables");
   if ((e = cudaMalloc(&ctx->d_jump, jump.size() * 8)) != cudaSuccess) return bail(e, "cudaMalloc tables");
   cudaMemcpy(ctx->d_sobol, sob.data(), sob.size() * 4, cudaMemcpyHostToDevice);
@@ -2249,6 +2270,7 @@ int mpc_create(const mpc_options_t* options, mpc_context_t** out) {
   ctx->live_bytes = sob.size() * 4 + jump.size() * 8;
   ctx->tabs.sobol = static_cast<const uint32_t*>(ctx->d_sobol);
   ctx->tabs.jump = static_cast<const uint64_t*>(ctx->d_jump);
+  ctx->tabs.lane_jump = ctx->tabs.jump + lane_at;
   *out = ctx;
   return MPC_OK;
 }

@@ -191,3 +191,26 @@ def test_headline_full_size_against_oracle(backend):
         a, b = backend.price(r32), backend.price(r64)
         assert abs(b.price - ref.price) <= 1e-10 * ref.price, (kw["model"], b.price, ref.price)
         assert abs(a.price - ref.price) < 0.05 * ref.stderr, (kw["model"], a.price, ref.price, ref.stderr)
+
+
+@pytest.mark.parametrize("n_paths,threads,kw", [
+    (1366, 1, {}),                                                # the path starts just pass one 4,096-position block
+    (4097, 1, dict(jump_intensity=0.0)),                          # no chain: one path past a block
+    (4096, 1, dict(jump_intensity=20.0, jump_mean=0.01)),         # nearly every path jumps: three positions a path
+    (4099, 2, dict(jump_intensity=1e-18)),                        # exp(-lambda T) rounds to 1: no path jumps
+    (6001, 3, dict(jump_intensity=800.0, jump_mean=1e-4, jump_volatility=1e-4)),  # exp(-lambda T) underflows: all do
+    (360_001, 1, dict(jump_intensity=0.4)),                       # more blocks than one scan of the chain takes
+    (700_003, 64, {}),                                            # many chunks of a few blocks
+])
+def test_merton_stream_blocks_per_path(backend, n_paths, threads, kw):
+    """Path starts across the device's stream blocks, per path against the
+    oracle; twice, since a call leaves its counters ready for the next."""
+
+    r = req("european_call", **{**MERTON, **dict(n_paths=n_paths, seed=77, n_threads=threads), **kw})
+    _, ref = O.price_paths(r)
+    for _ in range(2):
+        got = backend.price_paths(r)
+        assert np.allclose(got, ref, rtol=1e-11, atol=1e-12), np.max(np.abs(got - ref))
+    a, b = backend.price(r), O.price(r)
+    assert abs(a.price - b.price) <= 1e-11 * abs(b.price) + 1e-15
+    assert abs(a.stderr - b.stderr) <= 1e-9 * abs(b.stderr) + 1e-15
