@@ -1,7 +1,7 @@
 """Builds ``montepath_b200/lib/libmontepath_cuda.so`` for sm_100a with nvcc.
 
 Usage: ``python -m montepath_b200.build`` (or ``__graft_entry__.build()``).
-The three translation units compile in parallel and link into one shared
+The translation units compile in parallel and link into one shared
 library with the CUDA runtime linked statically, so the library loads on a
 machine without a GPU (calls then return MPC_E_NO_DEVICE).
 """
@@ -19,10 +19,23 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(OUT_DIR, "obj")
 LIBRARY = os.path.join(OUT_DIR, "libmontepath_cuda.so")
-SOURCES = ["mpc_kernels.cu", "mpc_runtime.cu", "mpc_server.cu", "mpc_peaks.cu", "mpc_noalloc.cu", "mpc_greeks.cu", "mpc_merton.cu"]
+SOURCES = [
+    "mpc_kernels.cu",
+    "mpc_plain_stream.cu",
+    "mpc_plain_lattice.cu",
+    "mpc_plain_sobol.cu",
+    "mpc_runtime.cu",
+    "mpc_server.cu",
+    "mpc_peaks.cu",
+    "mpc_noalloc.cu",
+    "mpc_greeks.cu",
+    "mpc_merton.cu",
+]
 HEADERS = [
     "mpc_device.cuh",
     "mpc_launch.h",
+    "mpc_models.cuh",
+    "mpc_plain.cuh",
     "mpc_runtime.h",
     "mpc_types.h",
     "sobol_directions.h",

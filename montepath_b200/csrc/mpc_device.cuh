@@ -56,6 +56,35 @@ __device__ __forceinline__ uint64_t xorshift_jump_uniform(const uint64_t* __rest
   return state;
 }
 
+// xorshift_jump for a whole warp (all 32 lanes call it together) whose lanes
+// start from one state and jump k = k0 + d draws, k0 lane 0's and d >= 0
+// small: the common k0 by the uniform jump, then every set bit of any d with
+// all lanes on the same table, whose 16-entry rows are one 128-byte line each.
+// Jumping lane by lane, one iteration touches a table per distinct bit.
+__device__ __forceinline__ uint64_t xorshift_jump_warp(const uint64_t* __restrict__ nibble, uint64_t state, uint64_t k) {
+  const uint64_t k0 = __shfl_sync(0xFFFFFFFFu, k, 0);
+  state = xorshift_jump_uniform(nibble, state, k0);
+  const uint64_t d = k - k0;
+  uint64_t any = ((uint64_t)__reduce_or_sync(0xFFFFFFFFu, (uint32_t)(d >> 32)) << 32) |
+                 __reduce_or_sync(0xFFFFFFFFu, (uint32_t)d);
+  while (any) {
+    const int b = __ffsll((long long)any) - 1;
+    const uint64_t y = gf2_apply(nibble + (size_t)b * 256, state);
+    if ((d >> b) & 1u) state = y;
+    any &= any - 1;
+  }
+  return state;
+}
+// The state `k` draws into the stream of `seed`, for all lanes of a warp at
+// once: by the shared jump when the lanes follow one stream forward, else
+// (a chunk edge inside the warp) lane by lane.
+__device__ __forceinline__ uint64_t xorshift_seek_warp(const uint64_t* __restrict__ nibble, uint64_t seed, uint64_t k) {
+  const uint64_t first = seed == 0 ? 0x9E3779B97F4A7C15ull : seed;  // MonteCarloRng replaces seed 0
+  // both shuffles before any test: every lane takes part in each
+  const uint64_t first0 = __shfl_sync(0xFFFFFFFFu, first, 0), k0 = __shfl_sync(0xFFFFFFFFu, k, 0);
+  return __all_sync(0xFFFFFFFFu, first == first0 && k >= k0) ? xorshift_jump_warp(nibble, first, k) : xorshift_jump(nibble, first, k);
+}
+
 // Sequential MonteCarloRng positioned at an arbitrary normal index.
 __device__ __forceinline__ float neg2_log_fast(float u);
 
@@ -93,7 +122,7 @@ struct XorshiftStream {
     double u2 = next_open01();
     double radius = sqrt(-2.0 * log(u1));
     double s, c;
-    sincos(6.283185307179586 * u2, &s, &c);
+    sincospi(2.0 * u2, &s, &c);  // exact argument reduction (the reference rounds 2 pi u2 first)
     cached = radius * s;
     has_cached = true;
     return radius * c;
@@ -357,6 +386,32 @@ __device__ __forceinline__ double icdf_f64(double p) {
   double num = mad(mad(mad(mad(mad(c0, q, c1), q, c2), q, c3), q, c4), q, c5);
   double den = mad(mad(mad(mad(d0, q, d1), q, d2), q, d3), q, 1.0);
   return -num / den;
+}
+
+// icdf_f64(sobol_unit_f64(x)) from the Sobol sample's bits.  The uniform and
+// its mirror 1 - u are the same expression of m = x >> 9 and of its 23-bit
+// complement, the rational is odd about 1/2 bit for bit, and the two tails
+// mirror each other, so the lower half serves both with the sign of bit 31.
+// `tail` holds the MPC_ICDF_TAIL values of the lower tail (icdf_f64 itself,
+// tabulated): evaluated in place, one lane of a warp in the tail (4.85% of the
+// samples, so four warps in five) makes all 32 wait for log, sqrt and a second
+// rational.  The centre's argument comes from the bits exactly: 2 m + 1 below
+// 2^52's exponent, less 2^52 + 2^23, times 2^-24.
+__device__ __forceinline__ double icdf_sobol_f64(const double* __restrict__ tail, uint32_t x) {
+  const double a0 = -3.969683028665376e1, a1 = 2.209460984245205e2, a2 = -2.759285104469687e2,
+               a3 = 1.38357751867269e2, a4 = -3.066479806614716e1, a5 = 2.506628277459239;
+  const double b0 = -5.447609879822406e1, b1 = 1.615858368580409e2, b2 = -1.556989798598866e2,
+               b3 = 6.680131188771972e1, b4 = -1.328068155288572e1;
+  const uint32_t xm = x ^ (uint32_t)((int32_t)x >> 31);
+  const uint32_t m = xm >> 9;
+  const double q = (__hiloint2double(0x43300000, (int)((xm >> 8) | 1u)) - 4503599635759104.0) * 5.9604644775390625e-08;
+  const double r = __dmul_rn(q, q);
+  auto mad = [](double acc, double y, double c) { return __dadd_rn(__dmul_rn(acc, y), c); };
+  const double num = __dmul_rn(mad(mad(mad(mad(mad(a0, r, a1), r, a2), r, a3), r, a4), r, a5), q);
+  const double den = mad(mad(mad(mad(mad(b0, r, b1), r, b2), r, b3), r, b4), r, 1.0);
+  double z = num / den;
+  if (m < MPC_ICDF_TAIL) z = __ldg(tail + m);
+  return __hiloint2double(__double2hiint(z) ^ (int)(x & 0x80000000u), __double2loint(z));
 }
 
 // --------------------------------------------------------------- Halton ---

@@ -8,10 +8,6 @@
 // list, so a single request, a heterogeneous book and a serving wave all use
 // the same launch.
 //
-// Plain path (FP64, one request per launch sequence): samples materialised
-// in HBM, a stepping kernel writing per-path payoffs (the contract of the
-// reference's mc_cuda_european_call_stepwise_v1), and a reduction kernel.
-//
 // Longstaff-Schwartz: one cooperative launch.  Paths are written date-major,
 // each date's ITM basis moments are reduced block -> grid (FP64), every block
 // solves the 4x4 normal equations redundantly after a bounded grid barrier,
@@ -27,6 +23,7 @@
 #include "../../include/montepath_cuda.h"
 #include "mpc_device.cuh"
 #include "mpc_launch.h"
+#include "mpc_models.cuh"
 #include "mpc_types.h"
 
 namespace mpc {
@@ -36,969 +33,6 @@ uint64_t kernel_launch_count() { return g_launches.load(); }
 void count_graph_launches(uint64_t kernels) { g_launches.fetch_add(kernels); }
 void discount_captured_launches(uint64_t kernels) { g_launches.fetch_sub(kernels); }
 static inline void count_launch() { g_launches.fetch_add(1); }
-
-enum Workload : int32_t {
-  W_EURO = 0,
-  W_ASIAN = 1,
-  W_DAO = 2,
-  W_UAO = 3,
-  W_LOOKBACK = 4,
-};
-
-struct SrcCtx {
-  const uint32_t* sobol;  // device lookup table (MPC_SOBOL_TABLE_WORDS words)
-  const uint64_t* jump;
-  uint32_t* win;          // shared-memory window of Sobol table rows (fused kernel), null elsewhere
-  const float4* icdf;     // shared-memory copy of the inverse-normal segments (fused kernel)
-};
-
-// Dimensions of the Sobol table rows staged in shared memory at a time, and
-// the row stride in words: kSobolWindow + 4 is 4 mod 32, so the 16 rows one
-// warp touches with a 128-bit load fall into two wavefronts.  The window
-// holds the 48 rows of the index's three low nibbles and one constant row:
-// a bit of the Owen-shuffled index depends only on the point's bits at and
-// above it (and the seed), so bits 12..31 of the shuffled index are the same
-// for every point of one aligned 4,096-point group, and the XOR of their five
-// nibble rows is one word per dimension.  The points a block runs together
-// (one iteration of a tile: at most 512 consecutive aligned units, the tile's
-// idle threads repeating the iteration's first unit) lie in one such group.
-// The output scramble's seed of a dimension, hash_combine(seed_g, dim),
-// depends on the block's seed and the dimension alone, so a last row holds
-// it for the window's dimensions: a quad reads its four seeds with one load.
-constexpr uint32_t kSobolWindow = 64;
-constexpr uint32_t kSobolRowStride = kSobolWindow + 4;
-constexpr uint32_t kSobolLowNibbles = 3;                        // nibble positions 0..2 staged per point
-constexpr uint32_t kSobolLowRows = 16 * kSobolLowNibbles;       // 48 rows
-constexpr uint32_t kSobolConstRow = kSobolLowRows;              // XOR of the upper nibble rows
-constexpr uint32_t kSobolSeedRow = kSobolLowRows + 1;           // output-scramble seed per dimension
-constexpr uint32_t kSobolWindowWords = (kSobolLowRows + 2) * kSobolRowStride;  // 13,600 bytes
-
-// Phi^-1(u) for a 23-bit midpoint uniform u from the segment table: v =
-// min(u, 1 - u) (exact) selects binade and one of 32 segments from its
-// exponent and top mantissa bits, the remaining 18 mantissa bits give the
-// position t in [0, 1/32) in the segment (they sit below 1.0's exponent as
-// they are, so no shift is needed), and the segment's cubic gives Phi^-1(v).
-// Defined for v in [2^-24, 1/2), which every 23-bit midpoint uniform meets.
-__device__ __forceinline__ float icdf_segments(const float4* __restrict__ seg, float u) {
-  const float v = fminf(u, 1.0f - u);
-  const uint32_t bits = __float_as_uint(v);
-  const uint32_t idx = (bits >> 18) - (103u << 5);  // (exponent - 103) * 32 + top 5 mantissa bits
-  const float t = __int_as_float((bits & 0x3FFFFu) | 0x3F800000u) - 1.0f;
-  const float4 c = seg[idx];
-  const float p = fmaf(fmaf(fmaf(c.w, t, c.z), t, c.y), t, c.x);
-  return u < 0.5f ? p : -p;
-}
-// icdf_segments(seg, sobol_unit_f32_bits(x)) from the Sobol sample's bits.
-// With m = x >> 9 the uniform is u = (m + 0.5) 2^-23, and its mirror 1 - u
-// is the same expression of the 23-bit complement of m, so
-// v = min(u, 1 - u) is built from x ^ (x >> 31, arithmetic): the complement
-// exactly when bit 31 (u > 1/2) is set, which also gives the result's sign.
-// Equal bit for bit to the two-step form, with no compare or select.
-__device__ __forceinline__ float icdf_sobol_bits(const float4* __restrict__ seg, uint32_t x) {
-  const uint32_t xm = x ^ (uint32_t)((int32_t)x >> 31);
-  const float v = __fsub_rn(__uint_as_float((xm >> 9) + 0x3F800000u), 0.99999994f);
-  const uint32_t bits = __float_as_uint(v);
-  const uint32_t idx = (bits >> 18) - (103u << 5);
-  const float t = __int_as_float((bits & 0x3FFFFu) | 0x3F800000u) - 1.0f;
-  const float4 c = seg[idx];
-  const float p = fmaf(fmaf(fmaf(c.w, t, c.z), t, c.y), t, c.x);
-  return __uint_as_float(__float_as_uint(p) ^ (x & 0x80000000u));
-}
-// Two samples at once: the floating-point steps as packed FP32 pairs
-// (FADD2 / FFMA2, each lane rounded exactly as the scalar operation), so the
-// pair equals two icdf_sobol_bits calls bit for bit.
-__device__ __forceinline__ float2 icdf_sobol_bits2(const float4* __restrict__ seg, uint32_t xa, uint32_t xb) {
-  const uint32_t ma = xa ^ (uint32_t)((int32_t)xa >> 31), mb = xb ^ (uint32_t)((int32_t)xb >> 31);
-  const float2 v = __fadd2_rn(make_float2(__uint_as_float((ma >> 9) + 0x3F800000u), __uint_as_float((mb >> 9) + 0x3F800000u)),
-                              make_float2(-0.99999994f, -0.99999994f));
-  const uint32_t ba = __float_as_uint(v.x), bb = __float_as_uint(v.y);
-  const float4 ca = seg[(ba >> 18) - (103u << 5)], cb = seg[(bb >> 18) - (103u << 5)];
-  const float2 t = __fadd2_rn(make_float2(__int_as_float((ba & 0x3FFFFu) | 0x3F800000u),
-                                          __int_as_float((bb & 0x3FFFFu) | 0x3F800000u)),
-                              make_float2(-1.0f, -1.0f));
-  float2 p = __ffma2_rn(make_float2(ca.w, cb.w), t, make_float2(ca.z, cb.z));
-  p = __ffma2_rn(p, t, make_float2(ca.y, cb.y));
-  p = __ffma2_rn(p, t, make_float2(ca.x, cb.x));
-  return make_float2(__uint_as_float(__float_as_uint(p.x) ^ (xa & 0x80000000u)),
-                     __uint_as_float(__float_as_uint(p.y) ^ (xb & 0x80000000u)));
-}
-
-// ------------------------------------------------------------- sources ----
-// A Source yields the samples of one unit (path or antithetic pair) by
-// dimension index.  n32/n64: standard normal in FP32 / FP64; u64: the raw
-// uniform (Merton's Poisson dimension).  Models announce each step's
-// dimensions with at_step(first, count) before sampling them; every thread
-// of a block makes the same at_step calls, which lets the Sobol source stage
-// its tables block-synchronously.
-template <int S>
-struct Source;
-
-template <>
-struct Source<SMP_COUNTER> {
-  uint32_t seed, unit;
-  template <bool FP64>
-  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx&, uint64_t u) {
-    seed = q.seed32;
-    unit = (uint32_t)u;
-  }
-  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ float n32(uint32_t d) { return counter_normal_f32(seed, unit, d); }
-  __device__ __forceinline__ double n64(uint32_t d) { return (double)counter_normal_f32(seed, unit, d); }
-  __device__ __forceinline__ double u64(uint32_t d) {
-    return (double)counter_open01(hash_u32(counter_mix(seed, unit, d, 0u)));
-  }
-  __device__ __forceinline__ float u32(uint32_t d) { return counter_open01(hash_u32(counter_mix(seed, unit, d, 0u))); }
-};
-
-// Scrambled Sobol with the per-point work hoisted: the Owen-shuffled index
-// and its nibble offsets depend only on (point, dimension group of 256), so
-// they are recomputed when a path crosses into the next group; per
-// dimension only the 8 table lookups and the output scramble remain.  The
-// values equal sobol_point() bit for bit.  Reads the [dim][q][v] layout from
-// global memory (generators and the FP64 plain path).
-template <>
-struct Source<SMP_SOBOL> {
-  const uint32_t* table;
-  uint32_t local, block_seed, group, seed_g, combine_g;
-  uint32_t off[8];
-  template <bool FP64>
-  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx& c, uint64_t u) {
-    table = c.sobol;
-    local = (uint32_t)(u & 0xFFFFu);
-    block_seed = q.seed32 + (uint32_t)(u >> 16) * 0x9E3779B9u;
-    group = 0xFFFFFFFFu;
-  }
-  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ uint32_t sample(uint32_t d) {
-    const uint32_t g = d / MPC_SOBOL_TABLE_DIMS;
-    if (g != group) {
-      group = g;
-      seed_g = block_seed + g;
-      const uint32_t shuffled = nested_uniform_scramble(local, seed_g);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) off[q] = q * 16 + ((shuffled >> (4 * q)) & 0xFu);
-      combine_g = 0x9e3779b9u + (seed_g << 6) + (seed_g >> 2);
-    }
-    const uint32_t dim = d & (MPC_SOBOL_TABLE_DIMS - 1);
-    const uint32_t* td = table + dim * 128;
-    uint32_t x = 0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) x ^= __ldg(td + off[q]);
-    return nested_uniform_scramble(x, seed_g ^ (dim + combine_g));  // hash_combine(seed_g, dim)
-  }
-  __device__ __forceinline__ float n32(uint32_t d) { return normcdfinvf(sobol_unit_f32(sample(d))); }
-  __device__ __forceinline__ float u32(uint32_t d) { return sobol_unit_f32(sample(d)); }
-  __device__ __forceinline__ double n64(uint32_t d) { return icdf_f64(sobol_unit_f64(sample(d))); }
-  __device__ __forceinline__ double u64(uint32_t d) { return sobol_unit_f64(sample(d)); }
-};
-
-template <>
-struct Source<SMP_HALTON> {
-  uint64_t index;
-  const uint32_t* primes;
-  const double* shifts;
-  template <bool FP64>
-  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx&, uint64_t u) {
-    index = u + 1;
-    primes = q.halton_primes;
-    shifts = q.halton_shifts;
-  }
-  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ double u64(uint32_t d) { return halton_shifted(index, __ldg(primes + d), __ldg(shifts + d)); }
-  __device__ __forceinline__ double n64(uint32_t d) { return icdf_f64(u64(d)); }
-  __device__ __forceinline__ float n32(uint32_t d) {
-    float u = fminf(fmaxf((float)u64(d), 5.9604645e-08f), 0.99999994f);
-    return normcdfinvf(u);
-  }
-  __device__ __forceinline__ float u32(uint32_t d) { return (float)u64(d); }
-};
-
-template <>
-struct Source<SMP_LHS> {
-  uint64_t point, n_paths;
-  const LhsDim* dims;
-  template <bool FP64>
-  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx&, uint64_t u) {
-    point = u;
-    n_paths = q.n_paths;
-    dims = q.lhs;
-  }
-  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ double u64(uint32_t d) {
-    LhsDim ld;
-    ld.multiplier = __ldg(&dims[d].multiplier);
-    ld.offset = __ldg(&dims[d].offset);
-    ld.jitter_seed = __ldg(&dims[d].jitter_seed);
-    return lhs_uniform(ld, point, n_paths);
-  }
-  __device__ __forceinline__ double n64(uint32_t d) { return icdf_f64(u64(d)); }
-  __device__ __forceinline__ float n32(uint32_t d) {
-    float u = fminf(fmaxf((float)u64(d), 5.9604645e-08f), 0.99999994f);
-    return normcdfinvf(u);
-  }
-  __device__ __forceinline__ float u32(uint32_t d) { return (float)u64(d); }
-};
-
-template <>
-struct Source<SMP_XORSHIFT> {
-  XorshiftStream st;
-  template <bool FP64>
-  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx& c, uint64_t u) {
-    uint64_t seed, local;
-    chunk_of(q, u, &seed, &local);
-    st.seek(c.jump, seed, local * q.normals_per_unit, !FP64);
-  }
-  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  // Sequential stream: dimensions must be requested in increasing order.
-  __device__ __forceinline__ float n32(uint32_t) { return st.normal_f32(); }
-  __device__ __forceinline__ double n64(uint32_t) { return st.normal_f64(); }
-  __device__ __forceinline__ double u64(uint32_t) { return st.next_open01(); }
-  __device__ __forceinline__ float u32(uint32_t) { return st.next_open01_f32(); }
-};
-
-// ------------------------------------------------ fused FP32 sources ---
-// The fused kernels draw their samples through FusedSource<SMP>::type:
-// the generic sources except for scrambled Sobol and the counter hash.
-
-// Scrambled Sobol for the fused kernels, bit-identical to Source<SMP_SOBOL>.
-// A block-synchronous window in shared memory holds, for each table row
-// r = 16 q + v of the three low nibble positions, the bit-reversed nibble
-// products of kSobolWindow consecutive dimensions, the constant row of the
-// upper positions and the output-scramble seeds, so one 128-bit load per row
-// serves four dimensions: a quad of dimensions costs 5 shared loads and 12
-// XORs instead of 32 loads.  XOR commutes with bit reversal, so the quad
-// holds brev(x) and the output scramble skips its first reversal.
-struct SobolQuad {
-  const uint32_t* rows_global;  // [128][256] bit-reversed rows
-  uint32_t* win;                // [kSobolLowRows + 2][kSobolRowStride] shared-memory window
-  const float4* icdf;           // inverse-normal segments in shared memory
-  uint32_t win_first;           // first dimension in the window (multiple of 4)
-  uint32_t local, block_seed, group, quad;
-  uint32_t rows[kSobolLowNibbles];  // window word offset of this point's row per low nibble position
-  uint32_t x0, x1, x2, x3;      // reversed products of the dimensions of `quad`
-  uint32_t s0, s1, s2, s3;      // their output-scramble seeds
-  template <bool FP64>
-  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx& c, uint64_t u) {
-    rows_global = c.sobol + MPC_SOBOL_NIBBLE_WORDS;
-    win = c.win;
-    icdf = c.icdf;
-    win_first = 0xFFFFFFFFu;
-    local = (uint32_t)(u & 0xFFFFu);
-    block_seed = q.seed32 + (uint32_t)(u >> 16) * 0x9E3779B9u;
-    group = 0xFFFFFFFFu;
-    quad = 0xFFFFFFFFu;
-  }
-  // Block-synchronous: restages the window at d0 rounded down to a multiple
-  // of 4 when [d0, d0 + count) is not inside it.  Requires
-  // count <= kSobolWindow - 3 so that the step fits the aligned window, and
-  // every point the block runs together in one aligned 4,096-point group, so
-  // that the constant row is theirs.  The low
-  // rows are 16-byte asynchronous global-to-shared transfers (four dimensions
-  // of one row each; an aligned quad never crosses the 256-dimension wrap),
-  // all in flight at once while the constant row is computed, then one wait.
-  __device__ __forceinline__ void at_step(uint32_t d0, uint32_t count) {
-    if (win_first != 0xFFFFFFFFu && d0 >= win_first && d0 + count <= win_first + kSobolWindow) return;
-    __syncthreads();
-    const uint32_t w0 = d0 & ~3u;
-    constexpr uint32_t kQuadsPerRow = kSobolWindow / 4;
-    const uint32_t win_s = (uint32_t)__cvta_generic_to_shared(win);
-    for (uint32_t i = threadIdx.x; i < kSobolLowRows * kQuadsPerRow; i += blockDim.x) {
-      const uint32_t row = i / kQuadsPerRow, j = 4 * (i % kQuadsPerRow);
-      const uint32_t* src = rows_global + row * MPC_SOBOL_TABLE_DIMS + ((w0 + j) & (MPC_SOBOL_TABLE_DIMS - 1));
-      const uint32_t dst = win_s + 4u * (row * kSobolRowStride + j);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-    }
-    for (uint32_t j = threadIdx.x; j < kSobolWindow; j += blockDim.x) {
-      const uint32_t d = w0 + j;
-      const uint32_t sg = block_seed + d / MPC_SOBOL_TABLE_DIMS;
-      // bits 12..31 of the shuffled index of this block's points (its bits
-      // below 12 do not reach them)
-      const uint32_t hi = nested_uniform_scramble(local & 0xF000u, sg);
-      const uint32_t dm = d & (MPC_SOBOL_TABLE_DIMS - 1);
-      uint32_t c = 0;
-#pragma unroll
-      for (int k = kSobolLowNibbles; k < 8; ++k)
-        c ^= __ldg(rows_global + (16u * k + ((hi >> (4 * k)) & 0xFu)) * MPC_SOBOL_TABLE_DIMS + dm);
-      win[kSobolConstRow * kSobolRowStride + j] = c;
-      win[kSobolSeedRow * kSobolRowStride + j] = hash_combine(sg, dm);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    win_first = w0;
-  }
-  // Loads the quad of dimensions [d0, d0 + 4), d0 a multiple of 4 inside
-  // the window (the chunked model loops call it directly).
-  __device__ __forceinline__ void quad_load(uint32_t d0) {
-    const uint32_t g = d0 / MPC_SOBOL_TABLE_DIMS;
-    if (g != group) {
-      group = g;
-      const uint32_t shuffled = nested_uniform_scramble(local, block_seed + g);
-#pragma unroll
-      for (int k = 0; k < (int)kSobolLowNibbles; ++k) rows[k] = (16u * k + ((shuffled >> (4 * k)) & 0xFu)) * kSobolRowStride;
-    }
-    quad = d0 >> 2;
-    const uint32_t* base = win + (d0 - win_first);
-    const uint4 sd = *reinterpret_cast<const uint4*>(base + kSobolSeedRow * kSobolRowStride);
-    s0 = sd.x;
-    s1 = sd.y;
-    s2 = sd.z;
-    s3 = sd.w;
-    uint4 a = *reinterpret_cast<const uint4*>(base + kSobolConstRow * kSobolRowStride);
-#pragma unroll
-    for (int k = 0; k < (int)kSobolLowNibbles; ++k) {
-      const uint4 b = *reinterpret_cast<const uint4*>(base + rows[k]);
-      a.x ^= b.x;
-      a.y ^= b.y;
-      a.z ^= b.z;
-      a.w ^= b.w;
-    }
-    x0 = a.x;
-    x1 = a.y;
-    x2 = a.z;
-    x3 = a.w;
-  }
-  // Scrambled value of dimension d0 + K of the quad loaded at d0.
-  template <int K>
-  __device__ __forceinline__ uint32_t take(uint32_t) const {
-    return __brev(lk_permute(K == 0 ? x0 : K == 1 ? x1 : K == 2 ? x2 : x3, K == 0 ? s0 : K == 1 ? s1 : K == 2 ? s2 : s3));
-  }
-  template <int K>
-  __device__ __forceinline__ float take_u(uint32_t d0) const {
-    return sobol_unit_f32_bits(take<K>(d0));
-  }
-  template <int K>
-  __device__ __forceinline__ float take_n(uint32_t d0) const {
-    return icdf_sobol_bits(icdf, take<K>(d0));
-  }
-  template <int K0, int K1>
-  __device__ __forceinline__ float2 take_n2(uint32_t d0) const {
-    return icdf_sobol_bits2(icdf, take<K0>(d0), take<K1>(d0));
-  }
-  __device__ __forceinline__ uint32_t sample(uint32_t d) {
-    if ((d >> 2) != quad) quad_load(d & ~3u);
-    const uint32_t k = d & 3u;
-    return __brev(lk_permute((k & 2u) ? ((k & 1u) ? x3 : x2) : ((k & 1u) ? x1 : x0),
-                             (k & 2u) ? ((k & 1u) ? s3 : s2) : ((k & 1u) ? s1 : s0)));
-  }
-  __device__ __forceinline__ float u32(uint32_t d) { return sobol_unit_f32_bits(sample(d)); }
-  __device__ __forceinline__ float n32(uint32_t d) { return icdf_sobol_bits(icdf, sample(d)); }
-  __device__ __forceinline__ double u64(uint32_t d) { return sobol_unit_f64(sample(d)); }
-  __device__ __forceinline__ double n64(uint32_t d) { return icdf_f64(u64(d)); }
-};
-
-// Counter-hash normals for the fused kernels: the reference's u32 hashes
-// with the short FP32 transform (counter_normal_fast).
-template <bool HWCOS>
-struct CounterFastT {
-  uint32_t seed, unit;
-  template <bool FP64>
-  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx&, uint64_t u) {
-    seed = q.seed32;
-    unit = (uint32_t)u;
-  }
-  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ float n32(uint32_t d) { return counter_normal_fast<HWCOS>(seed, unit, d); }
-  __device__ __forceinline__ float u32(uint32_t d) {
-    return counter_open01_fast(hash_u32(counter_mix(seed, unit, d, 0u)));
-  }
-  __device__ __forceinline__ double n64(uint32_t d) { return (double)counter_normal_f32(seed, unit, d); }
-  __device__ __forceinline__ double u64(uint32_t d) {
-    return (double)counter_open01(hash_u32(counter_mix(seed, unit, d, 0u)));
-  }
-};
-
-// Sources with the explicit-quad interface (quad_load / take_n / take_u).
-template <class S>
-constexpr bool kQuadSource = false;
-template <>
-constexpr bool kQuadSource<SobolQuad> = true;
-
-template <int SMP>
-struct FusedSource {
-  using type = Source<SMP>;
-};
-template <>
-struct FusedSource<SMP_SOBOL> {
-  using type = SobolQuad;
-};
-template <>
-struct FusedSource<SMP_COUNTER> {
-  using type = CounterFastT<false>;
-};
-// Per family: the single-asset GBM families (one normal per step, the MUFU
-// pipe about a third busy) take the hardware cosine; the others keep the
-// polynomial.
-template <int FAM, int SMP>
-struct FusedUnitSource {
-  using type = typename FusedSource<SMP>::type;
-};
-template <int FAM>
-struct FusedUnitSource<FAM, SMP_COUNTER> {
-  using type = CounterFastT<FAM == FAM_GBM_STEP || FAM == FAM_GBM_TERMINAL>;
-};
-
-// Reads materialised samples [dim][unit] (FP64 plain path).
-struct BufSource {
-  const double* buf;
-  uint64_t n_units, unit;
-  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ double n64(uint32_t d) { return buf[(uint64_t)d * n_units + unit]; }
-  __device__ __forceinline__ double u64(uint32_t d) { return buf[(uint64_t)d * n_units + unit]; }
-  __device__ __forceinline__ float n32(uint32_t d) { return (float)n64(d); }
-  __device__ __forceinline__ float u32(uint32_t d) { return (float)u64(d); }
-};
-
-template <class Real, class Src>
-__device__ __forceinline__ Real normal(Src& s, uint32_t d) {
-  if constexpr (sizeof(Real) == 4)
-    return s.n32(d);
-  else
-    return s.n64(d);
-}
-
-template <class Real>
-__device__ __forceinline__ Real ex(Real x) {
-  if constexpr (sizeof(Real) == 4)
-    return __expf(x);
-  else
-    return exp(x);
-}
-__device__ __forceinline__ float sqrt_approx(float x) {
-  float y;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-template <class Real>
-__device__ __forceinline__ Real sq_root(Real x) {
-  if constexpr (sizeof(Real) == 4)
-    return sqrt_approx(x);
-  else
-    return sqrt(x);
-}
-
-// sample_poisson by inversion with the uniform supplied (cpu.rs:932-953),
-// entered only when u > exp(-mean) (at least one jump); p0 = exp(-mean) is
-// precomputed on the host.
-__device__ __forceinline__ uint32_t poisson_tail(double u, double mean, double p0) {
-  double prob = p0, cum = p0;
-  uint32_t k = 0;
-  while (u > cum && k < 4095u) {
-    ++k;
-    prob *= mean / (double)k;
-    cum += prob;
-  }
-  return k;
-}
-
-// ------------------------------------------------------- Brownian bridge ---
-// fill_step_normals_from_inputs (cpu.rs:5964-5981) as a streaming walk: the
-// reference fills w[0..n] op by op and then differences it; here the same
-// ops run in the same (depth-first) order, but only the right endpoints still
-// needed stay on a small stack, and each leaf yields the next step's
-// increment (w[s] - w[s-1]) / sqrt(dt) at once.  Input dimensions are drawn in
-// increasing order (0 = W(T), then one per op), every thread of a request
-// runs the same event sequence, so block-synchronous sources stay in lockstep.
-// FP64 keeps the reference's two-rounding products and left-to-right sums.
-template <class Real>
-struct BridgeWalk {
-  Real stack[kBridgeDepth];
-  Real w_left;
-  uint32_t sp, ev, op, dim;
-
-  __device__ __forceinline__ static Real mid(Real lw, Real wl, Real rw, Real wr, Real sd, Real z) {
-    if constexpr (sizeof(Real) == 8)
-      return __dadd_rn(__dadd_rn(__dmul_rn(lw, wl), __dmul_rn(rw, wr)), __dmul_rn(sd, z));
-    else
-      return lw * wl + rw * wr + sd * z;
-  }
-  template <class Src>
-  __device__ __forceinline__ void begin(const DevReq& q, Src& src) {
-    src.at_step(0, 1);
-    const Real z0 = normal<Real>(src, 0);
-    if constexpr (sizeof(Real) == 8)
-      stack[0] = __dmul_rn(q.bridge_sqrt_t, z0);
-    else
-      stack[0] = (Real)q.bridge_sqrt_t * z0;
-    sp = 1;
-    w_left = (Real)0;
-    ev = 0;
-    op = 0;
-    dim = 1;
-  }
-  // The increment of the next step (the host checked the program: it ends
-  // every op run with a leaf and never needs more than kBridgeDepth values).
-  template <class Src>
-  __device__ __forceinline__ Real next(const DevReq& q, Src& src) {
-    for (;;) {
-      const uint32_t is_op = (__ldg(q.bridge_events + (ev >> 5)) >> (ev & 31)) & 1u;
-      ++ev;
-      if (!is_op) break;
-      const double* o = q.bridge_ops + 3 * op;
-      ++op;
-      src.at_step(dim, 1);
-      const Real z = normal<Real>(src, dim);
-      ++dim;
-      const Real wr = stack[sp - 1];
-      stack[sp] = mid((Real)__ldg(o), w_left, (Real)__ldg(o + 1), wr, (Real)__ldg(o + 2), z);
-      ++sp;
-    }
-    --sp;
-    const Real wr = stack[sp];
-    Real inc;
-    if constexpr (sizeof(Real) == 8)
-      inc = __dmul_rn(__dsub_rn(wr, w_left), q.bridge_inv_sqrt_dt);
-    else
-      inc = (wr - w_left) * (Real)q.bridge_inv_sqrt_dt;
-    w_left = wr;
-    return inc;
-  }
-};
-
-// ------------------------------------------------------------- models -----
-// GBM stepwise with the payoff observer of workload W (cpu.rs:6443-6591,
-// 7973-8009, 8324-8354; up-and-out mirrors down-and-out).  FP32 compares the
-// barrier in log space; FP64 compares exp(log S) with the barrier as the
-// reference does.
-template <class Real, int W, class Src, bool BRIDGE = false>
-__device__ __forceinline__ void unit_gbm_step(const DevReq& q, Src& src, double& pay, double& ctl) {
-  const Real drift = (Real)q.drift_dt, vol = (Real)q.vol_dt, kk = (Real)q.k, disc = (Real)q.discount;
-  const Real lbar = (Real)q.log_barrier, bar = (Real)q.barrier;
-  const bool anti = q.anti != 0;
-  Real ls0 = (Real)q.log_s0, ls1 = ls0;
-  Real acc0 = (W == W_LOOKBACK) ? (Real)q.s0 : (Real)0, acc1 = acc0;
-  bool ko0 = (W == W_DAO && q.s0 <= q.barrier) || (W == W_UAO && q.s0 >= q.barrier), ko1 = ko0;
-  const uint32_t n = q.n_steps;
-  auto advance = [&](const Real z) {
-    ls0 += drift + vol * z;
-    if (anti) ls1 += drift - vol * z;
-    if constexpr (W == W_ASIAN) {
-      acc0 += ex<Real>(ls0);
-      if (anti) acc1 += ex<Real>(ls1);
-    } else if constexpr (W == W_LOOKBACK) {
-      acc0 = acc0 > ex<Real>(ls0) ? acc0 : ex<Real>(ls0);
-      if (anti) acc1 = acc1 > ex<Real>(ls1) ? acc1 : ex<Real>(ls1);
-    } else if constexpr (W == W_DAO) {
-      if constexpr (sizeof(Real) == 4) {
-        ko0 |= ls0 <= lbar;
-        if (anti) ko1 |= ls1 <= lbar;
-      } else {
-        ko0 |= ex<Real>(ls0) <= bar;
-        if (anti) ko1 |= ex<Real>(ls1) <= bar;
-      }
-    } else if constexpr (W == W_UAO) {
-      if constexpr (sizeof(Real) == 4) {
-        ko0 |= ls0 >= lbar;
-        if (anti) ko1 |= ls1 >= lbar;
-      } else {
-        ko0 |= ex<Real>(ls0) >= bar;
-        if (anti) ko1 |= ex<Real>(ls1) >= bar;
-      }
-    }
-  };
-  uint32_t s = 0;
-  if constexpr (BRIDGE) {  // increments from the Brownian bridge over the inputs
-    BridgeWalk<Real> bw;
-    bw.begin(q, src);
-    for (; s < n; ++s) advance(bw.next(q, src));
-  } else if constexpr (kQuadSource<Src>) {
-    for (; s + 4 <= n; s += 4) {  // four steps per quad of dimensions
-      src.at_step(s, 4);
-      src.quad_load(s);
-      const float2 z01 = src.template take_n2<0, 1>(s), z23 = src.template take_n2<2, 3>(s);
-      advance(z01.x);
-      advance(z01.y);
-      advance(z23.x);
-      advance(z23.y);
-    }
-  }
-  for (; s < n; ++s) {
-    src.at_step(s, 1);
-    advance(normal<Real>(src, s));
-  }
-  auto payoff = [&](Real ls, Real acc, bool ko) -> Real {
-    Real v;
-    if constexpr (W == W_ASIAN) {
-      if constexpr (sizeof(Real) == 4)
-        v = acc * (Real)(1.0 / (double)n) - kk;
-      else
-        v = acc / (Real)n - kk;
-    } else if constexpr (W == W_LOOKBACK) {
-      v = acc - kk;
-    } else {
-      v = ex<Real>(ls) - kk;
-      if (ko) v = 0;
-    }
-    return (v > (Real)0 ? v : (Real)0) * disc;
-  };
-  Real p0 = payoff(ls0, acc0, ko0);
-  if (anti) {
-    Real p1 = payoff(ls1, acc1, ko1);
-    pay = 0.5 * ((double)p0 + (double)p1);
-  } else {
-    pay = (double)p0;
-  }
-  ctl = (double)(disc * ex<Real>(ls0));
-}
-
-// GBM terminal European (european_call_payoff_from_shock, cpu.rs:7773-7783).
-template <class Real, class Src>
-__device__ __forceinline__ void unit_gbm_terminal(const DevReq& q, Src& src, double& pay, double& ctl) {
-  src.at_step(0, 1);
-  const Real z = normal<Real>(src, 0);
-  const Real s0 = (Real)q.s0, drift = (Real)q.drift_dt, vol = (Real)q.vol_dt, kk = (Real)q.k,
-             disc = (Real)q.discount;
-  Real st = s0 * ex<Real>(drift + vol * z);
-  Real p = (st - kk > (Real)0 ? st - kk : (Real)0) * disc;
-  if (q.anti) {
-    Real sb = s0 * ex<Real>(drift + vol * (-z));
-    Real pb = (sb - kk > (Real)0 ? sb - kk : (Real)0) * disc;
-    pay = 0.5 * ((double)p + (double)pb);
-  } else {
-    pay = (double)p;
-  }
-  ctl = (double)(disc * st);
-}
-
-// Heston Euler with the variance floored after every step (heston_path_terminal, cpu.rs:8667-8686).
-template <class Real, class Src>
-__device__ __forceinline__ void unit_heston(const DevReq& q, Src& src, double& pay, double& ctl) {
-  const Real kappa = (Real)q.kappa, theta = (Real)q.theta, xi = (Real)q.xi, rho = (Real)q.rho,
-             rho_perp = (Real)q.rho_perp, dt = (Real)q.dt, sqdt = (Real)q.sqrt_dt, rate = (Real)q.rate;
-  const bool anti = q.anti != 0;
-  Real ls0 = (Real)q.log_s0, ls1 = ls0, v0 = (Real)q.v0, v1 = v0;
-  const uint32_t n = q.n_steps;
-  // FP32 path: the same update with the step constants folded on the host
-  // (rate dt, dt / 2, kappa dt, kappa theta dt, xi sqrt(dt)) and FMAs; the
-  // variance is floored after every step and starts >= 0 (validated), so it
-  // needs no floor before use.  The FP64 path keeps the reference's form.
-  // (Rearranged into fewer instructions -- the drift of all steps folded into
-  // the start, 1 - kappa dt, rho sqrt(dt) -- it measured 2.5% slower: two
-  // dependent FMAs on the log-price per step instead of one add.)
-  const float c_rdt = (float)(q.rate * q.dt), c_hdt = (float)(0.5 * q.dt), c_kdt = (float)(q.kappa * q.dt),
-              c_ktdt = (float)(q.kappa * q.theta * q.dt), c_xsq = (float)(q.xi * q.sqrt_dt);
-  auto step_f32 = [&](float& ls, float& v, const float zv, const float zi) {
-    const float sv = sqrt_approx(v);
-    const float zp = fmaf(rho, zv, rho_perp * zi);
-    ls += fmaf(sv * sqdt, zp, fmaf(-c_hdt, v, c_rdt));
-    const float vn = fmaf(c_xsq * sv, zv, v + fmaf(-c_kdt, v, c_ktdt));
-    v = vn > 0.0f ? vn : 0.0f;
-  };
-  auto step = [&](const Real zv, const Real zi) {
-    if constexpr (sizeof(Real) == 4) {
-      step_f32(ls0, v0, zv, zi);
-      if (anti) step_f32(ls1, v1, -zv, -zi);
-      return;
-    }
-    {
-      Real vp = v0 > (Real)0 ? v0 : (Real)0;
-      Real sv = sq_root<Real>(vp);
-      Real zp = rho * zv + rho_perp * zi;
-      ls0 += (rate - (Real)0.5 * vp) * dt + sv * sqdt * zp;
-      v0 = v0 + kappa * (theta - vp) * dt + xi * sv * sqdt * zv;
-      v0 = v0 > (Real)0 ? v0 : (Real)0;
-    }
-    if (anti) {
-      Real vp = v1 > (Real)0 ? v1 : (Real)0;
-      Real sv = sq_root<Real>(vp);
-      Real zp = rho * (-zv) + rho_perp * (-zi);
-      ls1 += (rate - (Real)0.5 * vp) * dt + sv * sqdt * zp;
-      v1 = v1 + kappa * (theta - vp) * dt + xi * sv * sqdt * (-zv);
-      v1 = v1 > (Real)0 ? v1 : (Real)0;
-    }
-  };
-  uint32_t s = 0;
-  if constexpr (kQuadSource<Src>) {
-    for (; s + 2 <= n; s += 2) {  // two steps per quad: dimensions 2s .. 2s + 3
-      const uint32_t d0 = 2 * s;
-      src.at_step(d0, 4);
-      src.quad_load(d0);
-      const float2 z01 = src.template take_n2<0, 1>(d0), z23 = src.template take_n2<2, 3>(d0);
-      step(z01.x, z01.y);
-      step(z23.x, z23.y);
-    }
-  }
-  for (; s < n; ++s) {
-    src.at_step(2 * s, 2);
-    const Real zv = normal<Real>(src, 2 * s);
-    const Real zi = normal<Real>(src, 2 * s + 1);
-    step(zv, zi);
-  }
-  const Real kk = (Real)q.k, disc = (Real)q.discount;
-  Real st = ex<Real>(ls0);
-  Real p = (st - kk > (Real)0 ? st - kk : (Real)0) * disc;
-  if (anti) {
-    Real sb = ex<Real>(ls1);
-    Real pb = (sb - kk > (Real)0 ? sb - kk : (Real)0) * disc;
-    pay = 0.5 * ((double)p + (double)pb);
-  } else {
-    pay = (double)p;
-  }
-  ctl = (double)(st * disc);
-}
-
-// Merton: stepwise extension (z, u, z_J per step) and the reference terminal
-// form (cpu.rs:6408-6441) with dims (z, u, z_J).
-template <class Real, bool STEP, class Src>
-__device__ __forceinline__ void unit_merton(const DevReq& q, Src& src, double& pay, double& ctl) {
-  const Real drift = (Real)q.drift_dt, vol = (Real)q.vol_dt, jm = (Real)q.jump_mean, jv = (Real)q.jump_vol;
-  Real ls = (Real)q.log_s0;
-  const uint32_t n = STEP ? q.n_steps : 1;
-  uint32_t s0 = 0;
-  // The FP32 Sobol path adds the deterministic drift of all n steps to the
-  // start (only the terminal log-price is read), so a step is one FMA.
-  if constexpr (kQuadSource<Src>) ls = (float)(q.log_s0 + q.drift_dt * (double)n);
-  if constexpr (kQuadSource<Src>) {
-    // four steps per three quads: step k of the chunk uses dimensions
-    // d0 + 3k (z), d0 + 3k + 1 (Poisson uniform), d0 + 3k + 2 (jump normal)
-    // xu: the scrambled 32-bit Poisson sample; its top 23 bits against the
-    // integer thresholds give the jump count of sample_poisson exactly (the
-    // FP64 inversion only from four jumps on)
-    // (xu >> 9) >= m0 exactly when xu >= m0 << 9 (m0 < 2^23): the shift
-    // leaves the common no-jump case
-    const uint32_t pois_x0 = q.pois_m[0] << 9;
-    auto step = [&](const float z, const uint32_t xu, auto&& jump_normal) {
-      ls = fmaf(vol, z, ls);
-      if (xu >= pois_x0) {
-        const uint32_t mu = xu >> 9;
-        uint32_t jumps = 1u + (mu >= q.pois_m[1] ? 1u : 0u) + (mu >= q.pois_m[2] ? 1u : 0u) + (mu >= q.pois_m[3] ? 1u : 0u);
-        if (jumps == 4u) jumps = poisson_tail((double)sobol_unit_f32_bits(xu), q.lam_dt, q.lam_p0);
-        ls += (Real)jumps * jm + jv * sq_root<Real>((Real)jumps) * jump_normal();
-      }
-    };
-    for (; s0 + 4 <= n; s0 += 4) {
-      const uint32_t d0 = 3 * s0;
-      src.at_step(d0, 12);
-      src.quad_load(d0);
-      const float z0 = src.template take_n<0>(d0);
-      const uint32_t u0 = src.template take<1>(d0);
-      step(z0, u0, [&] { return src.template take_n<2>(d0); });
-      const float z1 = src.template take_n<3>(d0);
-      src.quad_load(d0 + 4);
-      const uint32_t u1 = src.template take<0>(d0 + 4);
-      step(z1, u1, [&] { return src.template take_n<1>(d0 + 4); });
-      const float z2 = src.template take_n<2>(d0 + 4);
-      const uint32_t u2 = src.template take<3>(d0 + 4);
-      src.quad_load(d0 + 8);
-      step(z2, u2, [&] { return src.template take_n<0>(d0 + 8); });
-      step(src.template take_n<1>(d0 + 8), src.template take<2>(d0 + 8),
-           [&] { return src.template take_n<3>(d0 + 8); });
-    }
-  }
-  for (uint32_t s = s0; s < n; ++s) {
-    src.at_step(3 * s, 3);
-    const Real z = normal<Real>(src, 3 * s);
-    uint32_t jumps;
-    if constexpr (sizeof(Real) == 4) {
-      const float u = src.u32(3 * s + 1);
-      jumps = u <= q.lam_p0_f ? 0u : poisson_tail((double)u, q.lam_dt, q.lam_p0);
-    } else {
-      const double u = src.u64(3 * s + 1);
-      jumps = u <= q.lam_p0 ? 0u : poisson_tail(u, q.lam_dt, q.lam_p0);
-    }
-    if constexpr (kQuadSource<Src>)
-      ls = fmaf(vol, z, ls);
-    else
-      ls += drift + vol * z;
-    if (jumps > 0) {
-      const Real zj = normal<Real>(src, 3 * s + 2);
-      ls += (Real)jumps * jm + jv * sq_root<Real>((Real)jumps) * zj;
-    }
-  }
-  const Real kk = (Real)q.k, disc = (Real)q.discount;
-  Real st = ex<Real>(ls);
-  pay = (double)((st - kk > (Real)0 ? st - kk : (Real)0) * disc);
-  ctl = (double)(st * disc);
-}
-
-// d-asset basket, terminal or stepwise (basket_terminal_payoff, cpu.rs:7616-7635),
-// for a compile-time asset count D: the Cholesky factor and per-asset step
-// constants are converted to Real once per unit and kept in registers, and
-// every asset loop unrolls without predicates.
-template <class Real, int D, class Src>
-__device__ __forceinline__ void unit_basket_d(const DevReq& q, Src& src, double& pay, double& ctl) {
-  const uint32_t n = q.n_steps;
-  const bool anti = q.anti != 0;
-  Real L[D][D], dr[D], vo[D], x0[D], x1[D];
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-    dr[a] = (Real)q.b_drift[a];
-    vo[a] = (Real)q.b_vol[a];
-    x0[a] = x1[a] = (Real)0;
-#pragma unroll
-    for (int b = 0; b <= a; ++b) L[a][b] = (Real)q.chol[a * D + b];
-  }
-  uint32_t dim = 0;
-  for (uint32_t s = 0; s < n; ++s) {
-    Real z[D];
-    src.at_step(dim, D);
-#pragma unroll
-    for (int a = 0; a < D; ++a) z[a] = normal<Real>(src, dim + a);
-    dim += D;
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-      Real zc = (Real)0;
-#pragma unroll
-      for (int b = 0; b <= a; ++b) zc += L[a][b] * z[b];
-      x0[a] += dr[a] + vo[a] * zc;
-      if (anti) x1[a] += dr[a] + vo[a] * (-zc);
-    }
-  }
-  Real b0 = 0, b1 = 0;
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-    b0 += (Real)q.weights[a] * ((Real)q.spots[a] * ex<Real>(x0[a]));
-    if (anti) b1 += (Real)q.weights[a] * ((Real)q.spots[a] * ex<Real>(x1[a]));
-  }
-  const Real kk = (Real)q.k, disc = (Real)q.discount;
-  Real p = (b0 - kk > (Real)0 ? b0 - kk : (Real)0) * disc;
-  if (anti) {
-    Real pb = (b1 - kk > (Real)0 ? b1 - kk : (Real)0) * disc;
-    pay = 0.5 * ((double)p + (double)pb);
-  } else {
-    pay = (double)p;
-  }
-  ctl = (double)(b0 * disc);
-}
-
-template <class Real, class Src>
-__device__ __forceinline__ void unit_basket(const DevReq& q, Src& src, double& pay, double& ctl) {
-  switch (q.n_assets) {
-    case 1:
-      unit_basket_d<Real, 1>(q, src, pay, ctl);
-      break;
-    case 2:
-      unit_basket_d<Real, 2>(q, src, pay, ctl);
-      break;
-    case 3:
-      unit_basket_d<Real, 3>(q, src, pay, ctl);
-      break;
-    case 4:
-      unit_basket_d<Real, 4>(q, src, pay, ctl);
-      break;
-    case 5:
-      unit_basket_d<Real, 5>(q, src, pay, ctl);
-      break;
-    case 6:
-      unit_basket_d<Real, 6>(q, src, pay, ctl);
-      break;
-    case 7:
-      unit_basket_d<Real, 7>(q, src, pay, ctl);
-      break;
-    default:
-      unit_basket_d<Real, 8>(q, src, pay, ctl);
-      break;
-  }
-}
-
-// Coupled MLMC level of the arithmetic Asian (cpu.rs:6641-6894): level 0 is
-// the plain Asian with the base steps; level l couples M fine normals per
-// coarse step with a coarse path driven by sum(z)/sqrt(M).
-template <class Real, class Src>
-__device__ __forceinline__ void unit_mlmc(const DevReq& q, Src& src, double& pay, double& ctl) {
-  const Real kk = (Real)q.k, disc = (Real)q.discount;
-  ctl = 0.0;
-  if (q.level == 0) {
-    const Real drift = (Real)q.f_drift, vol = (Real)q.f_vol;
-    Real ls = (Real)q.log_s0, acc = 0;
-    for (uint32_t s = 0; s < q.n_steps; ++s) {
-      src.at_step(s, 1);
-      ls += drift + vol * normal<Real>(src, s);
-      acc += ex<Real>(ls);
-    }
-    Real avg;
-    if constexpr (sizeof(Real) == 4)
-      avg = acc * (Real)q.inv_fine;
-    else
-      avg = acc / (Real)q.n_steps;
-    pay = (double)((avg - kk > (Real)0 ? avg - kk : (Real)0) * disc);
-    return;
-  }
-  const Real fd = (Real)q.f_drift, fv = (Real)q.f_vol, cd = (Real)q.c_drift, cv = (Real)q.c_vol;
-  const uint32_t M = q.refinement;
-  Real fl = (Real)q.log_s0, cl = fl, fs = 0, cs = 0;
-  uint32_t j = 0;
-  for (uint64_t c = 0; c < q.coarse_steps; ++c) {
-    Real zsum = 0;
-    for (uint32_t m = 0; m < M; ++m) {
-      src.at_step(j, 1);  // one dimension at a time: M may exceed what a window step holds
-      const Real z = normal<Real>(src, j++);
-      zsum += z;
-      fl += fd + fv * z;
-      fs += ex<Real>(fl);
-    }
-    Real zc;
-    if constexpr (sizeof(Real) == 4)
-      zc = zsum * (Real)q.inv_sqrt_m;
-    else
-      zc = zsum / sqrt((double)M);
-    cl += cd + cv * zc;
-    cs += ex<Real>(cl);
-  }
-  Real fa, ca;
-  if constexpr (sizeof(Real) == 4) {
-    fa = fs * (Real)q.inv_fine;
-    ca = cs * (Real)q.inv_coarse;
-  } else {
-    fa = fs / (Real)q.n_steps;
-    ca = cs / (Real)q.coarse_steps;
-  }
-  Real pf = (fa - kk > (Real)0 ? fa - kk : (Real)0) * disc;
-  Real pc = (ca - kk > (Real)0 ? ca - kk : (Real)0) * disc;
-  pay = (double)pf - (double)pc;
-}
-
-template <class Real, int FAM, class Src>
-__device__ __forceinline__ void run_family(const DevReq& q, Src& src, double& p, double& c) {
-  if constexpr (FAM == FAM_GBM_BRIDGE) {
-    switch (q.workload) {
-      case W_ASIAN:
-        unit_gbm_step<Real, W_ASIAN, Src, true>(q, src, p, c);
-        break;
-      case W_DAO:
-        unit_gbm_step<Real, W_DAO, Src, true>(q, src, p, c);
-        break;
-      case W_UAO:
-        unit_gbm_step<Real, W_UAO, Src, true>(q, src, p, c);
-        break;
-      case W_LOOKBACK:
-        unit_gbm_step<Real, W_LOOKBACK, Src, true>(q, src, p, c);
-        break;
-      default:
-        unit_gbm_step<Real, W_EURO, Src, true>(q, src, p, c);
-        break;
-    }
-  } else if constexpr (FAM == FAM_GBM_STEP) {
-    switch (q.workload) {
-      case W_ASIAN:
-        unit_gbm_step<Real, W_ASIAN>(q, src, p, c);
-        break;
-      case W_DAO:
-        unit_gbm_step<Real, W_DAO>(q, src, p, c);
-        break;
-      case W_UAO:
-        unit_gbm_step<Real, W_UAO>(q, src, p, c);
-        break;
-      case W_LOOKBACK:
-        unit_gbm_step<Real, W_LOOKBACK>(q, src, p, c);
-        break;
-      default:
-        unit_gbm_step<Real, W_EURO>(q, src, p, c);
-        break;
-    }
-  } else if constexpr (FAM == FAM_GBM_TERMINAL) {
-    unit_gbm_terminal<Real>(q, src, p, c);
-  } else if constexpr (FAM == FAM_HESTON) {
-    unit_heston<Real>(q, src, p, c);
-  } else if constexpr (FAM == FAM_MERTON_STEP) {
-    unit_merton<Real, true>(q, src, p, c);
-  } else if constexpr (FAM == FAM_MERTON_TERMINAL) {
-    unit_merton<Real, false>(q, src, p, c);
-  } else if constexpr (FAM == FAM_BASKET) {
-    unit_basket<Real>(q, src, p, c);
-  } else {
-    unit_mlmc<Real>(q, src, p, c);
-  }
-}
 
 template <int FAM, int SMP>
 __device__ __forceinline__ void fused_unit(const DevReq& q, const SrcCtx& ctx, uint64_t u, double& p, double& c) {
@@ -1042,62 +76,6 @@ __device__ __forceinline__ void fused_unit_any(const DevReq& q, const SrcCtx& ct
         p = c = 0.0;
       }
       break;
-  }
-}
-
-// ----------------------------------------------------- block reduction ----
-constexpr int kFusedBlock = 256;
-constexpr int kWarps = kFusedBlock / 32;
-// The fused pricing kernel runs 128-, 256- or 512-thread blocks (the
-// autotuner's choice); its launch bounds are written for 512 threads.
-constexpr int kMaxFusedBlock = 512;
-constexpr int kMaxWarps = kMaxFusedBlock / 32;
-
-// Reduces v[0..4] over the block in a fixed order; result valid in thread 0.
-// The leading barrier keeps a previous call's reader of `red` safe, so calls
-// may follow each other directly.
-__device__ __forceinline__ void block_reduce5(double v[5], double (*red)[5]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < 5; ++i) v[i] = warp_sum(v[i]);
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < 5; ++i) red[warp][i] = v[i];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int warps = (blockDim.x + 31) >> 5;
-    for (int i = 0; i < 5; ++i) {
-      double s = 0.0;
-      for (int w = 0; w < warps; ++w) s += red[w][i];
-      v[i] = s;
-    }
-  }
-}
-
-// Sums the request's tile partials in tile order (strided per thread, then a
-// fixed block tree) into q.moments.  Called by the block that finished the
-// request's last tile.
-__device__ void finalize_request(DevReq& q, double (*red)[5]) {
-  double acc[5] = {0, 0, 0, 0, 0};
-  double cnt = 0.0;
-  for (uint32_t t = threadIdx.x; t < q.n_tiles; t += blockDim.x) {
-    const double* pt = q.partials + (size_t)t * MPC_MOMENTS;
-    cnt += __ldcg(pt + 0);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) acc[i] += __ldcg(pt + 1 + i);
-  }
-  double v[5] = {acc[0], acc[1], acc[2], acc[3], acc[4]};
-  block_reduce5(v, red);
-  double c6[5] = {cnt, 0, 0, 0, 0};
-  block_reduce5(c6, red);
-  if (threadIdx.x == 0) {
-    q.moments[0] = c6[0];
-    for (int i = 0; i < 5; ++i) q.moments[1 + i] = v[i];
-    q.moments[6] = 0.0;
-    q.moments[7] = 0.0;
-    *q.tiles_done = 0u;  // reusable without a memset
   }
 }
 
@@ -2102,160 +1080,6 @@ cudaError_t launch_basket_scenarios(const DevReq* d_req, uint32_t n_tiles, uint3
     default:
       return cudaErrorInvalidValue;
   }
-}
-
-// ------------------------------------------------------ FP64 plain path ---
-__device__ __forceinline__ bool is_uniform_dim(const DevReq& q, uint32_t d) {
-  return (q.family == FAM_MERTON_STEP || q.family == FAM_MERTON_TERMINAL) && (d % 3u) == 1u;
-}
-
-template <int SMP>
-__global__ void __launch_bounds__(256) plain_generate_kernel(DevReq q, double* __restrict__ buf, SrcCtx ctx) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint32_t dims = (uint32_t)q.normals_per_unit;
-  for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < q.n_units; u += stride) {
-    Source<SMP> src;
-    src.template begin<true>(q, ctx, u);
-    for (uint32_t d = 0; d < dims; ++d) buf[(uint64_t)d * q.n_units + u] = is_uniform_dim(q, d) ? src.u64(d) : src.n64(d);
-  }
-}
-
-cudaError_t launch_plain_generate(const DevReq& q, double* d_buf, int sampler, const DeviceTables& tabs,
-                                  cudaStream_t stream) {
-  SrcCtx ctx{tabs.sobol, tabs.jump, nullptr};
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  uint64_t want = (q.n_units + 255) / 256;
-  int grid = (int)(want < (uint64_t)sms * 8 ? want : (uint64_t)sms * 8);
-  if (grid < 1) grid = 1;
-  switch (sampler) {
-    case SMP_XORSHIFT:
-      plain_generate_kernel<SMP_XORSHIFT><<<grid, 256, 0, stream>>>(q, d_buf, ctx);
-      break;
-    case SMP_HALTON:
-      plain_generate_kernel<SMP_HALTON><<<grid, 256, 0, stream>>>(q, d_buf, ctx);
-      break;
-    case SMP_LHS:
-      plain_generate_kernel<SMP_LHS><<<grid, 256, 0, stream>>>(q, d_buf, ctx);
-      break;
-    case SMP_SOBOL:
-      plain_generate_kernel<SMP_SOBOL><<<grid, 256, 0, stream>>>(q, d_buf, ctx);
-      break;
-    case SMP_COUNTER:
-      plain_generate_kernel<SMP_COUNTER><<<grid, 256, 0, stream>>>(q, d_buf, ctx);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  count_launch();
-  return cudaGetLastError();
-}
-
-template <int FAM>
-__global__ void __launch_bounds__(256) plain_simulate_kernel(const DevReq* __restrict__ qp,
-                                                             const double* __restrict__ buf,
-                                                             double* __restrict__ payoff,
-                                                             double* __restrict__ control) {
-  const DevReq& q = *qp;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < q.n_units; u += stride) {
-    BufSource src{buf, q.n_units, u};
-    double p, c;
-    run_family<double, FAM>(q, src, p, c);
-    payoff[u] = p;
-    if (control) control[u] = c;
-  }
-}
-
-cudaError_t launch_plain_simulate(const DevReq& q, const DevReq* d_req, const double* d_buf, double* d_payoff,
-                                  double* d_control, cudaStream_t stream) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  uint64_t want = (q.n_units + 255) / 256;
-  int grid = (int)(want < (uint64_t)sms * 8 ? want : (uint64_t)sms * 8);
-  if (grid < 1) grid = 1;
-  switch (q.family) {
-    case FAM_GBM_STEP:
-      plain_simulate_kernel<FAM_GBM_STEP><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-    case FAM_GBM_TERMINAL:
-      plain_simulate_kernel<FAM_GBM_TERMINAL><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-    case FAM_HESTON:
-      plain_simulate_kernel<FAM_HESTON><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-    case FAM_MERTON_STEP:
-      plain_simulate_kernel<FAM_MERTON_STEP><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-    case FAM_MERTON_TERMINAL:
-      plain_simulate_kernel<FAM_MERTON_TERMINAL><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-    case FAM_BASKET:
-      plain_simulate_kernel<FAM_BASKET><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-    case FAM_GBM_BRIDGE:
-      plain_simulate_kernel<FAM_GBM_BRIDGE><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-    default:
-      plain_simulate_kernel<FAM_MLMC_LEVEL><<<grid, 256, 0, stream>>>(d_req, d_buf, d_payoff, d_control);
-      break;
-  }
-  count_launch();
-  return cudaGetLastError();
-}
-
-// Deterministic FP64 reduction of the payoff (and control) buffers in tiles
-// of q.tile_units, finalized by the last tile.
-__global__ void __launch_bounds__(kFusedBlock) plain_reduce_kernel(DevReq* __restrict__ qp,
-                                                                   const double* __restrict__ payoff,
-                                                                   const double* __restrict__ control) {
-  __shared__ double red[kWarps][5];
-  __shared__ int s_last;
-  DevReq& q = *qp;
-  for (uint32_t t = blockIdx.x; t < q.n_tiles; t += gridDim.x) {
-    const uint64_t first = (uint64_t)t * q.tile_units;
-    const uint64_t last = min(first + (uint64_t)q.tile_units, q.n_units);
-    double v[5] = {0, 0, 0, 0, 0};
-    for (uint64_t u = first + threadIdx.x; u < last; u += blockDim.x) {
-      const double p = payoff[u];
-      v[0] += p;
-      v[1] += p * p;
-      if (control) {
-        const double c = control[u];
-        v[2] += c;
-        v[3] += c * c;
-        v[4] += p * c;
-      }
-    }
-    block_reduce5(v, red);
-    if (threadIdx.x == 0) {
-      double* pt = q.partials + (size_t)t * MPC_MOMENTS;
-      pt[0] = (double)(last - first);
-      for (int i = 0; i < 5; ++i) pt[1 + i] = v[i];
-      __threadfence();
-      s_last = (atomicAdd(q.tiles_done, 1u) == q.n_tiles - 1) ? 1 : 0;
-    }
-    __syncthreads();
-    if (s_last) {
-      __threadfence();
-      finalize_request(q, red);
-    }
-    __syncthreads();
-  }
-}
-
-cudaError_t launch_plain_reduce(const DevReq* d_req, const double* d_payoff, const double* d_control,
-                                uint64_t n_units, uint32_t n_tiles, cudaStream_t stream) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int grid = (int)(n_tiles < (uint32_t)sms * 4 ? n_tiles : (uint32_t)sms * 4);
-  if (grid < 1) grid = 1;
-  plain_reduce_kernel<<<grid, kFusedBlock, 0, stream>>>(const_cast<DevReq*>(d_req), d_payoff, d_control);
-  count_launch();
-  return cudaGetLastError();
 }
 
 // ---------------------------------------- reference v1 kernel contract ----

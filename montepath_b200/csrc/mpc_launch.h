@@ -13,6 +13,7 @@ struct DeviceTables {
   const uint32_t* sobol;  // [256][8][16] nibble tables
   const uint64_t* jump;   // [64][16][16] xorshift jump nibble tables
   const uint64_t* lane_jump;  // [16][16][32] (q, v, lane): v << 4q jumped kMertonRun * lane draws; contexts only
+  const double* icdf_tail;    // [MPC_ICDF_TAIL] lower tail of the FP64 inverse normal; contexts only
 };
 
 // Fused FP32 path: one persistent launch over a tile work list.  All
@@ -53,13 +54,17 @@ struct LoopArgs {
 cudaError_t launch_serve_loop(const LoopArgs& a, const DeviceTables& tabs, int grid, cudaStream_t stream);
 int serve_loop_blocks_per_sm();
 
-// FP64 plain path: materialise samples, simulate into a payoff buffer, reduce.
-cudaError_t launch_plain_generate(const DevReq& q, double* d_buf, int sampler, const DeviceTables& tabs,
-                                  cudaStream_t stream);
-cudaError_t launch_plain_simulate(const DevReq& q, const DevReq* d_req, const double* d_buf, double* d_payoff,
-                                  double* d_control, cudaStream_t stream);
-cudaError_t launch_plain_reduce(const DevReq* d_req, const double* d_payoff, const double* d_control,
-                                uint64_t n_units, uint32_t n_tiles, cudaStream_t stream);
+// FP64 plain path: one launch per request (q.n_tiles blocks of `block`
+// threads, 32 to 128), moments written to q.moments by the last block;
+// *q.tiles_done is zero before and after.
+cudaError_t launch_plain(const DevReq& q, int sampler, const DeviceTables& tabs, int block, cudaStream_t stream);
+// The same for pseudorandom stepwise GBM with `lanes` (2 to 32, a power of two)
+// threads per path, block = q.tile_units * lanes; each lane holds at most
+// kPlainSplitNormals normals.
+constexpr uint32_t kPlainSplitNormals = 32;
+cudaError_t launch_plain_split(const DevReq& q, const DeviceTables& tabs, int block, uint32_t lanes, cudaStream_t stream);
+// Fills the MPC_ICDF_TAIL values of DeviceTables::icdf_tail.
+cudaError_t launch_icdf_tail(double* d_out, cudaStream_t stream);
 
 // Reference kernel contract mc_cuda_european_call_stepwise_v1.
 cudaError_t launch_european_call_stepwise_v1(const double* normals, double* payoffs, int32_t n_paths,

@@ -72,6 +72,7 @@ struct mpc_context {
   mpc::DeviceTables tabs{};
   void* d_sobol = nullptr;
   void* d_jump = nullptr;
+  void* d_icdf_tail = nullptr;
   uint64_t budget = 0;
   uint64_t live_bytes = 0;
   uint64_t peak_bytes = 0;

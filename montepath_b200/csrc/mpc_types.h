@@ -14,6 +14,8 @@
 #define MPC_ICDF_SEGMENTS (23 * 32)
 #define MPC_ICDF_OFFSET (2 * MPC_SOBOL_NIBBLE_WORDS)
 #define MPC_SOBOL_TABLE_WORDS (MPC_ICDF_OFFSET + 4 * MPC_ICDF_SEGMENTS)
+// 23-bit midpoint uniforms in the lower tail of the inverse normal (u < 0.02425).
+#define MPC_ICDF_TAIL 203424u
 // Moments per tile / request: count, sum p, sum p^2, sum c, sum c^2, sum p*c (+2 pad).
 #define MPC_MOMENTS 8
 
