@@ -81,10 +81,12 @@ __device__ __forceinline__ void fused_unit_any(const DevReq& q, const SrcCtx& ct
 
 // --------------------------------------------------------- fused kernel ---
 // Resident blocks per SM the register allocation must allow: the
-// family-switching instance is the widest; the GBM and terminal families
-// with the counter-hash generator are long serial chains that want more warps.
+// family-switching instance is the widest; terminal paths on the counter hash
+// are one short chain that wants more warps (stepwise ones draw two normals at
+// a time and want the registers: 439 us with 40 of them, 375 us with 64, the
+// book's single-asset part).
 constexpr int fused_min_blocks(int fam, int smp) {
-  return fam < 0 ? 2 : ((fam == FAM_GBM_STEP || fam == FAM_GBM_TERMINAL) && smp == SMP_COUNTER ? 6 : 4);
+  return fam < 0 ? 2 : (fam == FAM_GBM_TERMINAL && smp == SMP_COUNTER ? 6 : 4);
 }
 // The same resident threads per SM (hence the same register budget per
 // thread) expressed in 512-thread blocks, for the launch bounds.
@@ -106,8 +108,8 @@ __device__ __forceinline__ uint64_t gf2_apply_shared(const uint64_t* table, uint
 // 2 * (idx / 2) draws, idx the unit's first normal in its chunk.
 template <int FAM>
 __device__ __forceinline__ void fused_unit_stream(const DevReq& q, uint64_t aligned, uint64_t idx, double& p, double& c) {
-  Source<SMP_XORSHIFT> src;
-  src.st.seek_aligned(aligned, idx, true);
+  XorshiftFast src;
+  src.start(aligned, idx);
   run_family<float, FAM>(q, src, p, c);
 }
 
@@ -119,9 +121,9 @@ __device__ __forceinline__ void fused_tile(const DevReq& sq, const SrcCtx& ctx, 
   double v[5] = {0, 0, 0, 0, 0};
   const bool cv = sq.cv != 0;
   double* per_unit = sq.per_unit;
-  // Every thread runs the same number of units so that block-synchronous
-  // sources stay in lockstep; a thread past the tile end repeats the first
-  // unit and discards it.
+  // Every thread runs the same number of units so that block- and
+  // warp-synchronous sources stay in lockstep; a thread past the tile end
+  // repeats the tile's last unit and discards it.
   const uint32_t iters = (uint32_t)((last - first + blockDim.x - 1) / blockDim.x);
   // Pseudorandom streams in a single-family kernel: a thread's units of one
   // tile lie blockDim units apart, so inside one chunk the next unit's
@@ -155,16 +157,19 @@ __device__ __forceinline__ void fused_tile(const DevReq& sq, const SrcCtx& ctx, 
   for (uint32_t it = 0; it < iters; ++it) {
     uint64_t u = first + threadIdx.x + (uint64_t)it * blockDim.x;
     const bool valid = u < last;
-    if (!valid) u = first + (uint64_t)it * blockDim.x;  // the iteration's first unit: same Sobol index bits 12..31
+    if (!valid) u = last - 1;  // a unit of the same iteration: same Sobol index bits 12..31, and not behind the warp's first
     double p, c;
     if constexpr (kStride) {
       uint64_t seed, local;
       chunk_of(sq, u, &seed, &local);
       const uint64_t idx = local * sq.normals_per_unit;
-      if (chained && valid && seed == prev_seed)
+      const bool jump = chained && valid && seed == prev_seed;
+      if (__all_sync(0xFFFFFFFFu, jump)) {
         aligned = gf2_apply_shared(stride_tab, aligned);
-      else
-        aligned = xorshift_jump(ctx.jump, XorshiftStream::first_state(seed), 2 * (idx >> 1));
+      } else {
+        const uint64_t sought = xorshift_seek_warp(ctx.jump, seed, 2 * (idx >> 1));
+        aligned = jump ? gf2_apply_shared(stride_tab, aligned) : sought;
+      }
       chained = valid;
       prev_seed = seed;
       fused_unit_stream<FAM>(sq, aligned, idx, p, c);
@@ -569,25 +574,35 @@ __device__ __forceinline__ void scen_gbm_step(const DevReq& q, Src& src, const f
   }
   const float lbar = (float)q.log_barrier;
   const uint32_t n = q.n_steps;
-  for (uint32_t st = 0; st < n; ++st) {
-    src.at_step(st, 1);
-    const float z = normal<float>(src, st);
+  auto advance = [&](const float z) {
 #pragma unroll
     for (int s = 0; s < kMaxScen; ++s) {
       if (s >= n_scen) break;
       ls[s] += drift[s] + vol[s] * z;
-      if constexpr (W == W_ASIAN) acc[s] += __expf(ls[s]);
-      else if constexpr (W == W_LOOKBACK) acc[s] = acc[s] > __expf(ls[s]) ? acc[s] : __expf(ls[s]);
+      if constexpr (W == W_ASIAN) acc[s] += ex<float>(ls[s]);
+      else if constexpr (W == W_LOOKBACK) acc[s] = acc[s] > ex<float>(ls[s]) ? acc[s] : ex<float>(ls[s]);
       else if constexpr (W == W_DAO) ko[s] |= ls[s] <= lbar;
       else if constexpr (W == W_UAO) ko[s] |= ls[s] >= lbar;
       if constexpr (ANTI) {
         ls2[s] += drift[s] - vol[s] * z;
-        if constexpr (W == W_ASIAN) acc2[s] += __expf(ls2[s]);
-        else if constexpr (W == W_LOOKBACK) acc2[s] = acc2[s] > __expf(ls2[s]) ? acc2[s] : __expf(ls2[s]);
+        if constexpr (W == W_ASIAN) acc2[s] += ex<float>(ls2[s]);
+        else if constexpr (W == W_LOOKBACK) acc2[s] = acc2[s] > ex<float>(ls2[s]) ? acc2[s] : ex<float>(ls2[s]);
         else if constexpr (W == W_DAO) ko2[s] |= ls2[s] <= lbar;
         else if constexpr (W == W_UAO) ko2[s] |= ls2[s] >= lbar;
       }
     }
+  };
+  uint32_t st = 0;
+  if constexpr (kPairSource<Src>) {
+    for (; st + 2 <= n; st += 2) {
+      const float2 z = src.n32x2(st);
+      advance(z.x);
+      advance(z.y);
+    }
+  }
+  for (; st < n; ++st) {
+    src.at_step(st, 1);
+    advance(normal<float>(src, st));
   }
   const float kk = (float)q.k, inv_n = (float)(1.0 / (double)n);
   auto payoff = [&](float l, float a, bool out, float disc) {
@@ -595,7 +610,7 @@ __device__ __forceinline__ void scen_gbm_step(const DevReq& q, Src& src, const f
     if constexpr (W == W_ASIAN) v = a * inv_n - kk;
     else if constexpr (W == W_LOOKBACK) v = a - kk;
     else {
-      v = __expf(l) - kk;
+      v = ex<float>(l) - kk;
       if (out) v = 0.0f;
     }
     return (v > 0.0f ? v : 0.0f) * disc;
@@ -605,7 +620,7 @@ __device__ __forceinline__ void scen_gbm_step(const DevReq& q, Src& src, const f
     const float disc = __ldg(sp + 4 * kMaxScen + s);
     pay[s] = payoff(ls[s], acc[s], ko[s], disc);
     if constexpr (ANTI) pay2[s] = payoff(ls2[s], acc2[s], ko2[s], disc);
-    if constexpr (TECH == kScenCv) ctl[s] = disc * __expf(ls[s]);
+    if constexpr (TECH == kScenCv) ctl[s] = disc * ex<float>(ls[s]);
   }
 }
 
@@ -619,10 +634,10 @@ __device__ __forceinline__ void scen_gbm_terminal(const DevReq& q, Src& src, con
   for (int s = 0; s < kMaxScen; ++s) {
     const float s0 = __ldg(sp + 1 * kMaxScen + s), drift = __ldg(sp + 2 * kMaxScen + s),
                 vol = __ldg(sp + 3 * kMaxScen + s), disc = __ldg(sp + 4 * kMaxScen + s);
-    const float st = s0 * __expf(drift + vol * z);
+    const float st = s0 * ex<float>(drift + vol * z);
     pay[s] = (st - kk > 0.0f ? st - kk : 0.0f) * disc;
     if constexpr (TECH == kScenAnti) {
-      const float sb = s0 * __expf(drift + vol * (-z));
+      const float sb = s0 * ex<float>(drift + vol * (-z));
       pay2[s] = (sb - kk > 0.0f ? sb - kk : 0.0f) * disc;
     }
     if constexpr (TECH == kScenCv) ctl[s] = disc * st;
@@ -659,9 +674,16 @@ __device__ __forceinline__ void scen_heston(const DevReq& q, Src& src, const flo
   };
   const uint32_t n = q.n_steps;
   for (uint32_t st = 0; st < n; ++st) {
-    src.at_step(2 * st, 2);
-    const float zv = normal<float>(src, 2 * st);
-    const float zi = normal<float>(src, 2 * st + 1);
+    float zv, zi;
+    if constexpr (kPairSource<Src>) {
+      const float2 z = src.n32x2(2 * st);
+      zv = z.x;
+      zi = z.y;
+    } else {
+      src.at_step(2 * st, 2);
+      zv = normal<float>(src, 2 * st);
+      zi = normal<float>(src, 2 * st + 1);
+    }
     const float zp = rho * zv + rho_perp * zi;
 #pragma unroll
     for (int s = 0; s < kMaxScen; ++s) {
@@ -674,10 +696,10 @@ __device__ __forceinline__ void scen_heston(const DevReq& q, Src& src, const flo
 #pragma unroll
   for (int s = 0; s < kMaxScen; ++s) {
     const float disc = __ldg(sp + 5 * kMaxScen + s);
-    const float stv = __expf(ls[s]);
+    const float stv = ex<float>(ls[s]);
     pay[s] = (stv - kk > 0.0f ? stv - kk : 0.0f) * disc;
     if constexpr (ANTI) {
-      const float sb = __expf(ls2[s]);
+      const float sb = ex<float>(ls2[s]);
       pay2[s] = (sb - kk > 0.0f ? sb - kk : 0.0f) * disc;
     }
     if constexpr (TECH == kScenCv) ctl[s] = stv * disc;
@@ -753,7 +775,7 @@ __global__ void __launch_bounds__(kFusedBlock, 2) scenario_kernel(const DevReq* 
     for (uint32_t it = 0; it < iters; ++it) {
       uint64_t u = first + threadIdx.x + (uint64_t)it * blockDim.x;
       const bool valid = u < last;
-      if (!valid) u = first + (uint64_t)it * blockDim.x;  // lockstep for block-synchronous sources; discarded below
+      if (!valid) u = last - 1;  // lockstep for block- and warp-synchronous sources; discarded below
       typename FusedUnitSource<FAM, SMP>::type src;  // the samples fused_unit<FAM, SMP> draws
       src.template begin<false>(sq, ctx, u);
       float pay[kMaxScen], pay2[kMaxScen], ctl[kMaxScen];
@@ -900,16 +922,7 @@ template <int D, class Src>
 __device__ __forceinline__ void scen_basket_d(const DevReq& q, Src& src, const BasketScen& legs,
                                               float pay[kBasketScen]) {
   float zs[D];
-#pragma unroll
-  for (int a = 0; a < D; ++a) zs[a] = 0.0f;
-  const uint32_t n = q.n_steps;
-  uint32_t dim = 0;
-  for (uint32_t st = 0; st < n; ++st) {
-    src.at_step(dim, D);
-#pragma unroll
-    for (int a = 0; a < D; ++a) zs[a] += normal<float>(src, dim + a);
-    dim += D;
-  }
+  sum_step_normals<float, D>(src, q.n_steps, zs);
   float w[D];
 #pragma unroll
   for (int a = 0; a < D; ++a) {
@@ -923,7 +936,7 @@ __device__ __forceinline__ void scen_basket_d(const DevReq& q, Src& src, const B
   for (int s = 0; s < kBasketScen; ++s) {
     float basket = 0.0f;
 #pragma unroll
-    for (int a = 0; a < D; ++a) basket += legs.wspot[s][a] * __expf(legs.log_drift[s][a] + legs.step_vol[s][a] * w[a]);
+    for (int a = 0; a < D; ++a) basket += legs.wspot[s][a] * ex<float>(legs.log_drift[s][a] + legs.step_vol[s][a] * w[a]);
     pay[s] = (basket - kk > 0.0f ? basket - kk : 0.0f) * legs.discount[s];
   }
 }
@@ -999,7 +1012,7 @@ __global__ void __launch_bounds__(kFusedBlock, 2) basket_scenario_kernel(const D
     for (uint32_t it = 0; it < iters; ++it) {
       uint64_t u = first + threadIdx.x + (uint64_t)it * blockDim.x;
       const bool valid = u < last;
-      if (!valid) u = first + (uint64_t)it * blockDim.x;  // lockstep for block-synchronous sources; discarded below
+      if (!valid) u = last - 1;  // lockstep for block- and warp-synchronous sources; discarded below
       typename FusedUnitSource<FAM_BASKET, SMP>::type src;  // the samples fused_unit<FAM_BASKET, SMP> draws
       src.template begin<false>(sq, ctx, u);
       float pay[kBasketScen];

@@ -241,8 +241,9 @@ struct Source<SMP_XORSHIFT> {
 };
 
 // ------------------------------------------------ fused FP32 sources ---
-// The fused kernels draw their samples through FusedSource<SMP>::type:
-// the generic sources except for scrambled Sobol and the counter hash.
+// The fused kernels draw their samples through FusedUnitSource<FAM, SMP>::type:
+// the generic sources except for scrambled Sobol, the counter hash and the
+// pseudorandom stream.
 
 // Scrambled Sobol for the fused kernels, bit-identical to Source<SMP_SOBOL>.
 // A block-synchronous window in shared memory holds, for each table row
@@ -403,24 +404,77 @@ struct SobolPlain {
   }
 };
 
-// Counter-hash normals for the fused kernels: the reference's u32 hashes
-// with the short FP32 transform (counter_normal_fast).
+// Counter-hash normals for the fused kernels: the reference's u32 hashes with
+// the short FP32 transform, two dimensions at a time where the model can.
 template <bool HWCOS>
 struct CounterFastT {
-  uint32_t seed, unit;
+  uint32_t seed, unit, base;
   template <bool FP64>
   __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx&, uint64_t u) {
     seed = q.seed32;
     unit = (uint32_t)u;
+    base = counter_mix(seed, unit, 0u, 0u);
   }
   __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
   __device__ __forceinline__ float n32(uint32_t d) { return counter_normal_fast<HWCOS>(seed, unit, d); }
+  __device__ __forceinline__ float2 n32x2(uint32_t d) {
+    return counter_normal_pair<HWCOS>(base ^ (d * 2891336453u), base ^ ((d + 1u) * 2891336453u));
+  }
   __device__ __forceinline__ float u32(uint32_t d) {
     return counter_open01_fast(hash_u32(counter_mix(seed, unit, d, 0u)));
   }
   __device__ __forceinline__ double n64(uint32_t d) { return (double)counter_normal_f32(seed, unit, d); }
   __device__ __forceinline__ double u64(uint32_t d) {
     return (double)counter_open01(hash_u32(counter_mix(seed, unit, d, 0u)));
+  }
+};
+
+// The MonteCarloRng stream for the fused kernels, a Box-Muller pair at a time:
+// no cached-normal branch per sample, and the sine branch a unit with an odd
+// start carries over stays in FP32.  Dimensions in increasing order.
+struct XorshiftFast {
+  XorshiftStream st;
+  float carry;
+  bool odd;  // the next normal is `carry`
+  __device__ __forceinline__ float2 pair() {
+    const float u1 = st.next_open01_f32(), u2 = st.next_open01_f32();
+    const float r = sqrt_ftz(neg2_log_fast(u1));
+    float s, c;
+    // hardware sine and cosine of 2 pi (u2 - 1/2) in [-pi, pi], where their
+    // documented error is 2^-21.4 absolute
+    __sincosf(6.28318548f * (u2 - 0.5f), &s, &c);
+    return make_float2(r * -c, r * -s);
+  }
+  // Starts from `aligned`, the state after 2 * (idx / 2) draws.
+  __device__ __forceinline__ void start(uint64_t aligned, uint64_t idx) {
+    st.state = aligned;
+    odd = (idx & 1) != 0;
+    carry = 0.0f;
+    if (odd) carry = pair().y;
+  }
+  template <bool FP64>
+  __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx& c, uint64_t u) {
+    uint64_t seed, local;
+    chunk_of(q, u, &seed, &local);
+    const uint64_t idx = local * q.normals_per_unit;
+    start(xorshift_seek_warp(c.jump, seed, 2 * (idx >> 1)), idx);
+  }
+  __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
+  __device__ __forceinline__ float n32(uint32_t) {
+    if (odd) {
+      odd = false;
+      return carry;
+    }
+    const float2 z = pair();
+    odd = true;
+    carry = z.y;
+    return z.x;
+  }
+  __device__ __forceinline__ float2 n32x2(uint32_t) {
+    const float2 z = pair();
+    const float2 out = odd ? make_float2(carry, z.x) : z;
+    carry = z.y;
+    return out;
   }
 };
 
@@ -432,28 +486,31 @@ constexpr bool kQuadSource<SobolQuad> = true;
 template <>
 constexpr bool kQuadSource<SobolPlain> = true;
 
-template <int SMP>
-struct FusedSource {
-  using type = Source<SMP>;
-};
+// Sources that give the normals of two consecutive dimensions at once (n32x2).
+template <class S>
+constexpr bool kPairSource = false;
+template <bool HWCOS>
+constexpr bool kPairSource<CounterFastT<HWCOS>> = true;
 template <>
-struct FusedSource<SMP_SOBOL> {
-  using type = SobolQuad;
-};
-template <>
-struct FusedSource<SMP_COUNTER> {
-  using type = CounterFastT<false>;
-};
-// Per family: the single-asset GBM families (one normal per step, the MUFU
-// pipe about a third busy) take the hardware cosine; the others keep the
-// polynomial.
+constexpr bool kPairSource<XorshiftFast> = true;
+
 template <int FAM, int SMP>
 struct FusedUnitSource {
-  using type = typename FusedSource<SMP>::type;
+  using type = Source<SMP>;
 };
+template <int FAM>
+struct FusedUnitSource<FAM, SMP_SOBOL> {
+  using type = SobolQuad;
+};
+// The single-asset GBM families (one normal per step, the MUFU pipe about a
+// third busy) take the hardware cosine; the others keep the polynomial.
 template <int FAM>
 struct FusedUnitSource<FAM, SMP_COUNTER> {
   using type = CounterFastT<FAM == FAM_GBM_STEP || FAM == FAM_GBM_TERMINAL>;
+};
+template <int FAM>
+struct FusedUnitSource<FAM, SMP_XORSHIFT> {
+  using type = XorshiftFast;
 };
 
 template <class Real, class Src>
@@ -466,10 +523,15 @@ __device__ __forceinline__ Real normal(Src& s, uint32_t d) {
 
 template <class Real>
 __device__ __forceinline__ Real ex(Real x) {
-  if constexpr (sizeof(Real) == 4)
-    return __expf(x);
-  else
+  if constexpr (sizeof(Real) == 4) {
+    // __expf without its denormal scaling (prices and discounted payoffs are
+    // far from it): the same value for every normal result
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+    return y;
+  } else {
     return exp(x);
+  }
 }
 __device__ __forceinline__ float sqrt_approx(float x) {
   float y;
@@ -618,6 +680,12 @@ __device__ __forceinline__ void unit_gbm_step(const DevReq& q, Src& src, double&
       advance(z23.x);
       advance(z23.y);
     }
+  } else if constexpr (kPairSource<Src>) {
+    for (; s + 2 <= n; s += 2) {
+      const float2 z = src.n32x2(s);
+      advance(z.x);
+      advance(z.y);
+    }
   }
   for (; s < n; ++s) {
     src.at_step(s, 1);
@@ -724,6 +792,11 @@ __device__ __forceinline__ void unit_heston(const DevReq& q, Src& src, double& p
       step(z01.x, z01.y);
       step(z23.x, z23.y);
     }
+  } else if constexpr (kPairSource<Src>) {
+    for (; s < n; ++s) {
+      const float2 z = src.n32x2(2 * s);
+      step(z.x, z.y);
+    }
   }
   for (; s < n; ++s) {
     src.at_step(2 * s, 2);
@@ -823,48 +896,59 @@ __device__ __forceinline__ void unit_merton(const DevReq& q, Src& src, double& p
   ctl = (double)(st * disc);
 }
 
+// Sums over n steps of a path's D normals per step.
+template <class Real, int D, class Src>
+__device__ __forceinline__ void sum_step_normals(Src& src, uint32_t n, Real zs[D]) {
+#pragma unroll
+  for (int a = 0; a < D; ++a) zs[a] = (Real)0;
+  uint32_t dim = 0, s = 0;
+  if constexpr (kPairSource<Src>) {
+    // two steps are D pairs whatever D's parity
+    for (; s + 2 <= n; s += 2) {
+#pragma unroll
+      for (int p = 0; p < D; ++p) {
+        const float2 z = src.n32x2(dim + 2 * p);
+        zs[(2 * p) % D] += z.x;
+        zs[(2 * p + 1) % D] += z.y;
+      }
+      dim += 2 * D;
+    }
+  }
+  for (; s < n; ++s) {
+    src.at_step(dim, D);
+#pragma unroll
+    for (int a = 0; a < D; ++a) zs[a] += normal<Real>(src, dim + a);
+    dim += D;
+  }
+}
+
 // d-asset basket, terminal or stepwise (basket_terminal_payoff, cpu.rs:7616-7635),
-// for a compile-time asset count D: the Cholesky factor and per-asset step
-// constants are converted to Real once per unit and kept in registers, and
-// every asset loop unrolls without predicates.
+// for a compile-time asset count D.  The payoff reads terminal values only and
+// the log returns are linear in the normals, so a path keeps the D sums of its
+// normals over the steps and correlates them once at the end:
+// sum_steps (drift + vol (L z)_a) = n drift + vol (L sum_steps z)_a.  A step is
+// then D normals and D adds; correlating every step cost D (D + 1) / 2 + 2 D
+// more and held the Cholesky factor in registers through the whole path (64
+// registers a thread: 356 bytes spilled with D up to 8).  1.6e9 normals of
+// 5-asset baskets: 3,829 us, 3,211 us so, 2,380 us with the normals in pairs.
 template <class Real, int D, class Src>
 __device__ __forceinline__ void unit_basket_d(const DevReq& q, Src& src, double& pay, double& ctl) {
   const uint32_t n = q.n_steps;
-  const bool anti = q.anti != 0;
-  Real L[D][D], dr[D], vo[D], x0[D], x1[D];
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-    dr[a] = (Real)q.b_drift[a];
-    vo[a] = (Real)q.b_vol[a];
-    x0[a] = x1[a] = (Real)0;
-#pragma unroll
-    for (int b = 0; b <= a; ++b) L[a][b] = (Real)q.chol[a * D + b];
-  }
-  uint32_t dim = 0;
-  for (uint32_t s = 0; s < n; ++s) {
-    Real z[D];
-    src.at_step(dim, D);
-#pragma unroll
-    for (int a = 0; a < D; ++a) z[a] = normal<Real>(src, dim + a);
-    dim += D;
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-      Real zc = (Real)0;
-#pragma unroll
-      for (int b = 0; b <= a; ++b) zc += L[a][b] * z[b];
-      x0[a] += dr[a] + vo[a] * zc;
-      if (anti) x1[a] += dr[a] + vo[a] * (-zc);
-    }
-  }
+  Real zs[D];
+  sum_step_normals<Real, D>(src, n, zs);
   Real b0 = 0, b1 = 0;
 #pragma unroll
   for (int a = 0; a < D; ++a) {
-    b0 += (Real)q.weights[a] * ((Real)q.spots[a] * ex<Real>(x0[a]));
-    if (anti) b1 += (Real)q.weights[a] * ((Real)q.spots[a] * ex<Real>(x1[a]));
+    Real w = (Real)0;
+#pragma unroll
+    for (int b = 0; b <= a; ++b) w += (Real)q.chol[a * D + b] * zs[b];
+    const Real drift = (Real)(q.b_drift[a] * (double)n), vol = (Real)q.b_vol[a];
+    b0 += (Real)q.weights[a] * ((Real)q.spots[a] * ex<Real>(drift + vol * w));
+    if (q.anti) b1 += (Real)q.weights[a] * ((Real)q.spots[a] * ex<Real>(drift - vol * w));
   }
   const Real kk = (Real)q.k, disc = (Real)q.discount;
   Real p = (b0 - kk > (Real)0 ? b0 - kk : (Real)0) * disc;
-  if (anti) {
+  if (q.anti) {
     Real pb = (b1 - kk > (Real)0 ? b1 - kk : (Real)0) * disc;
     pay = 0.5 * ((double)p + (double)pb);
   } else {
@@ -913,10 +997,21 @@ __device__ __forceinline__ void unit_mlmc(const DevReq& q, Src& src, double& pay
   if (q.level == 0) {
     const Real drift = (Real)q.f_drift, vol = (Real)q.f_vol;
     Real ls = (Real)q.log_s0, acc = 0;
-    for (uint32_t s = 0; s < q.n_steps; ++s) {
-      src.at_step(s, 1);
-      ls += drift + vol * normal<Real>(src, s);
+    auto advance = [&](const Real z) {
+      ls += drift + vol * z;
       acc += ex<Real>(ls);
+    };
+    uint32_t s = 0;
+    if constexpr (kPairSource<Src>) {
+      for (; s + 2 <= q.n_steps; s += 2) {
+        const float2 z = src.n32x2(s);
+        advance(z.x);
+        advance(z.y);
+      }
+    }
+    for (; s < q.n_steps; ++s) {
+      src.at_step(s, 1);
+      advance(normal<Real>(src, s));
     }
     Real avg;
     if constexpr (sizeof(Real) == 4)
@@ -932,12 +1027,22 @@ __device__ __forceinline__ void unit_mlmc(const DevReq& q, Src& src, double& pay
   uint32_t j = 0;
   for (uint64_t c = 0; c < q.coarse_steps; ++c) {
     Real zsum = 0;
-    for (uint32_t m = 0; m < M; ++m) {
-      src.at_step(j, 1);  // one dimension at a time: M may exceed what a window step holds
-      const Real z = normal<Real>(src, j++);
+    auto fine = [&](const Real z) {
       zsum += z;
       fl += fd + fv * z;
       fs += ex<Real>(fl);
+    };
+    uint32_t m = 0;
+    if constexpr (kPairSource<Src>) {
+      for (; m + 2 <= M; m += 2, j += 2) {
+        const float2 z = src.n32x2(j);
+        fine(z.x);
+        fine(z.y);
+      }
+    }
+    for (; m < M; ++m) {
+      src.at_step(j, 1);  // one dimension at a time: M may exceed what a window step holds
+      fine(normal<Real>(src, j++));
     }
     Real zc;
     if constexpr (sizeof(Real) == 4)

@@ -1,0 +1,43 @@
+"""Fused FP32 units that draw their normals two at a time, per path against
+the FP64 oracle on the same samples: odd and even steps (a last single
+normal), odd stream positions, every asset count of a basket, chunk edges
+inside a warp.  FP32 paths: the tolerance of the other FP32 per-path tests
+(steps of a log price of 4.6, last place 4.8e-7, at S of 100 to 200)."""
+
+import numpy as np
+import pytest
+
+from montepath_b200.requests import make_request
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    ("european_call", dict(method="stepwise")),
+    ("european_call", dict(model="heston", kappa=2.0, vol_of_vol=0.5, rho=-0.7)),
+    ("arithmetic_asian_call", dict(technique="antithetic")),
+    ("lookback_call", dict(technique="control_variate")),
+]
+
+
+def check(backend, workload, kw):
+    _, ref = O.price_paths(make_request(workload, dict(kw, precision="fp64_plain")))
+    got = backend.price_paths(make_request(workload, dict(kw, precision="fp32_path")))
+    assert np.allclose(got, ref, rtol=1e-3, atol=2e-3), float(np.max(np.abs(got - ref)))
+
+
+@pytest.mark.parametrize("workload,kw", CASES)
+@pytest.mark.parametrize("sampling", ["pseudorandom", "counter_hash"])
+@pytest.mark.parametrize("n_paths,n_steps,threads", [(1, 1, 1), (33, 2, 1), (515, 3, 1), (8003, 36, 4)])
+def test_units_by_pairs(backend, workload, kw, sampling, n_paths, n_steps, threads):
+    check(backend, workload, dict(kw, sampling=sampling, n_paths=n_paths, n_steps=n_steps, n_threads=threads, seed=13))
+
+
+@pytest.mark.parametrize("assets", range(1, 9))
+@pytest.mark.parametrize("n_steps", [1, 2, 5])
+@pytest.mark.parametrize("sampling,technique", [("pseudorandom", "standard"), ("counter_hash", "antithetic")])
+def test_baskets_by_pairs(backend, assets, n_steps, sampling, technique):
+    corr = [[1.0 if i == j else 0.25 for j in range(assets)] for i in range(assets)]
+    check(backend, "basket_call", dict(method="stepwise", n_steps=n_steps, n_paths=2001, seed=6, sampling=sampling,
+                                       technique=technique, spots=[90.0 + 4.0 * i for i in range(assets)],
+                                       sigmas=[0.15 + 0.03 * i for i in range(assets)], corr=corr))
