@@ -176,7 +176,7 @@ int run_scenario_legs(mpc_context* ctx, const std::vector<mpc_request_t>& legs, 
   const int slots = basket ? kBasketScen : kMaxScen;  // legs per tile partial
   const int technique = legs[0].technique;
   const int nm = basket ? 2 : scenario_moments(technique);  // moments per leg
-  float scen[kScenFields * kMaxScen];
+  ScenarioLegs scen{};
   for (int s = 0; s < kMaxScen && !basket; ++s) {
     const DevReq& q = preps[s < n_scen ? s : 0].q;
     float f[kScenFields];
@@ -191,7 +191,7 @@ int run_scenario_legs(mpc_context* ctx, const std::vector<mpc_request_t>& legs, 
                                     float(q.vol_dt),   float(q.discount), ko ? 1.0f : 0.0f};
       std::memcpy(f, v, sizeof(f));
     }
-    for (int k = 0; k < kScenFields; ++k) scen[k * kMaxScen + s] = f[k];
+    for (int k = 0; k < kScenFields; ++k) scen.f[k * kMaxScen + s] = f[k];
   }
   DevReq q = base.q;
   q.n_scen = uint32_t(n_scen);
@@ -199,45 +199,29 @@ int run_scenario_legs(mpc_context* ctx, const std::vector<mpc_request_t>& legs, 
   const uint64_t n_tiles = (q.n_units + q.tile_units - 1) / q.tile_units;
   if (n_tiles > (1ull << 31)) return fail(ctx, MPC_E_UNSUPPORTED, "too many tiles for one scenario launch");
   q.n_tiles = uint32_t(n_tiles);
-  // device layout: descriptor | leg parameters | partials | moments | counters (done, tile counter)
-  const size_t o_scen = 256 * ((sizeof(DevReq) + 255) / 256);
-  const size_t o_part = o_scen + 256;
-  const size_t o_mom = o_part + ((n_tiles * slots * nm * sizeof(double) + 255) / 256) * 256;
-  const size_t o_cnt = o_mom + ((size_t(slots) * nm * sizeof(double) + 255) / 256) * 256;
-  void* d = nullptr;
-  int st = scratch(ctx, "scenarios", o_cnt + 256, &d);
+  // one launch: the descriptor and the legs travel as kernel parameters, the
+  // moments come back through pinned memory, and the counters (tiles done,
+  // cursor, blocks gone) are zero when allocated and after every launch
+  void *d_part = nullptr, *d_cnt = nullptr, *pin = nullptr;
+  int st = scratch(ctx, "scenarios", n_tiles * slots * nm * sizeof(double), &d_part);
+  if (st == MPC_OK) st = scratch(ctx, "scenario_counters", 4 * sizeof(uint32_t), &d_cnt);
+  if (st == MPC_OK) st = pinned_staging(ctx, size_t(slots) * nm * sizeof(double), &pin);
   if (st != MPC_OK) return st;
-  uint8_t* base_ptr = static_cast<uint8_t*>(d);
-  q.scen = reinterpret_cast<const float*>(base_ptr + o_scen);
-  q.partials = reinterpret_cast<double*>(base_ptr + o_part);
-  q.moments = reinterpret_cast<double*>(base_ptr + o_mom);
-  q.tiles_done = reinterpret_cast<uint32_t*>(base_ptr + o_cnt);
+  q.partials = static_cast<double*>(d_part);
+  q.moments = static_cast<double*>(pin);
+  q.tiles_done = static_cast<uint32_t*>(d_cnt);
   q.per_unit = nullptr;
-  uint32_t* counter = q.tiles_done + 1;
-  double host_mom[kBasketScen * 5];
-  static_assert(kBasketScen >= kMaxScen, "moments buffer");
+  const double* host_mom = static_cast<const double*>(pin);
   auto fin = [&](cudaError_t e, const char* what) { return e == cudaSuccess ? MPC_OK : cuda_fail(ctx, e, what); };
-  if ((st = fin(cudaMemsetAsync(q.tiles_done, 0, 2 * sizeof(uint32_t), ctx->stream), "memset counters"))) return st;
-  if ((st = fin(cudaMemcpyAsync(base_ptr, &q, sizeof(q), cudaMemcpyHostToDevice, ctx->stream), "descriptor"))) return st;
-  if (!basket && (st = fin(cudaMemcpyAsync(base_ptr + o_scen, scen, sizeof(scen), cudaMemcpyHostToDevice, ctx->stream),
-                           "leg parameters")))
-    return st;
   const int occ = std::max(1, basket ? basket_scenario_max_blocks_per_sm(base.sampler)
                                      : scenario_max_blocks_per_sm(base.family, base.sampler, technique));
   const int grid = int(std::min<uint64_t>(n_tiles, uint64_t(ctx->sm_count) * occ));
   if ((st = fin(cudaEventRecord(ctx->ev_start, ctx->stream), "event"))) return st;
-  const DevReq* d_req = reinterpret_cast<const DevReq*>(base_ptr);
   const cudaError_t launched =
-      basket ? launch_basket_scenarios(d_req, q.n_tiles, counter, base.sampler, basket_legs(preps), ctx->tabs, grid,
-                                       ctx->stream)
-             : launch_scenarios(d_req, q.n_tiles, counter, base.family, base.sampler, technique, ctx->tabs, grid,
-                                ctx->stream);
+      basket ? launch_basket_scenarios(q, base.sampler, basket_legs(preps), ctx->tabs, grid, ctx->stream)
+             : launch_scenarios(q, scen, base.family, base.sampler, technique, ctx->tabs, grid, ctx->stream);
   if ((st = fin(launched, "scenario kernel"))) return st;
   if ((st = fin(cudaEventRecord(ctx->ev_stop, ctx->stream), "event"))) return st;
-  if ((st = fin(cudaMemcpyAsync(host_mom, q.moments, size_t(slots) * nm * sizeof(double), cudaMemcpyDeviceToHost,
-                                ctx->stream),
-                "moments")))
-    return st;
   if ((st = fin(cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize"))) return st;
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
@@ -345,19 +329,20 @@ extern "C" int mpc_greeks(mpc_context_t* ctx, const mpc_request_t* req, int esti
   a.fp64 = r.precision == MPC_PRECISION_FP64_PLAIN ? 1 : 0;
   const uint64_t want = (r.n_paths + 255) / 256;
   const uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(ctx->sm_count) * 8)));
-  void* d = nullptr;
-  // partials [grid][8] | totals [8] | counter
-  if ((st = scratch(ctx, "greeks", (size_t(grid) * 8 + 8) * sizeof(double) + 64, &d)) != MPC_OK) return finish(st);
-  a.partials = static_cast<double*>(d);
-  a.out = a.partials + size_t(grid) * 8;
-  a.done = reinterpret_cast<unsigned*>(a.out + 8);
-  double host[8];
-  GREEKS_CUDA(cudaMemsetAsync(a.done, 0, sizeof(unsigned), ctx->stream));
+  void *d_part = nullptr, *d_done = nullptr, *pin = nullptr;
+  // partials [grid][8]; a counter that is zero when allocated and after every
+  // launch; totals [8] written to pinned memory
+  if ((st = scratch(ctx, "greeks", size_t(grid) * 8 * sizeof(double), &d_part)) != MPC_OK) return finish(st);
+  if ((st = scratch(ctx, "greeks_done", 16, &d_done)) != MPC_OK) return finish(st);
+  if ((st = pinned_staging(ctx, 8 * sizeof(double), &pin)) != MPC_OK) return finish(st);
+  a.partials = static_cast<double*>(d_part);
+  a.out = static_cast<double*>(pin);
+  a.done = static_cast<unsigned*>(d_done);
+  const double* host = a.out;
   GREEKS_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
   cudaError_t e = launch_greeks_single_pass(a, grid, ctx->tabs, ctx->stream);
   if (e != cudaSuccess) return finish(cuda_fail(ctx, e, "single-pass Greeks kernel"));
   GREEKS_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
-  GREEKS_CUDA(cudaMemcpyAsync(host, a.out, sizeof(host), cudaMemcpyDeviceToHost, ctx->stream));
   GREEKS_CUDA(cudaStreamSynchronize(ctx->stream));
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);

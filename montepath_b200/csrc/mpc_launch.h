@@ -16,11 +16,25 @@ struct DeviceTables {
   const double* icdf_tail;    // [MPC_ICDF_TAIL] lower tail of the FP64 inverse normal; contexts only
 };
 
+// Work of one fused launch (a kernel parameter): up to kFusedInline requests
+// held in the parameter itself, or a tile list over descriptors in device
+// memory.  Tile t of an inline launch belongs to the request r with
+// first[r] <= t < first[r + 1].  `counter` is the work list's cursor, zero at
+// launch; an inline launch has two words there and leaves them zero.
+constexpr uint32_t kFusedInline = 4;
+struct FusedWork {
+  uint32_t n_tiles, n_inline;   // n_inline 0: reqs and tiles
+  uint32_t* counter;
+  const DevReq* reqs;
+  const Tile* tiles;
+  uint32_t first[kFusedInline + 4];
+  DevReq inl[kFusedInline];
+};
+
 // Fused FP32 path: one persistent launch over a tile work list.  All
-// requests in `reqs` must share `sampler`; `family` < 0 lets each tile switch
-// on its request's family (mixed batches).
-cudaError_t launch_fused(const DevReq* d_reqs, const Tile* d_tiles, uint32_t n_tiles, uint32_t* d_tile_counter,
-                         int family, int sampler, const DeviceTables& tabs, int grid, int block,
+// requests of the launch must share `sampler`; `family` < 0 lets each tile
+// switch on its request's family (mixed batches).
+cudaError_t launch_fused(const FusedWork& work, int family, int sampler, const DeviceTables& tabs, int grid, int block,
                          cudaStream_t stream);
 int fused_max_blocks_per_sm(int family, int sampler, int block);
 
@@ -124,22 +138,26 @@ constexpr uint32_t kLsmThreads = 512;
 // uint 4, the error code at uint 8 and its index at uint 10.
 constexpr size_t kLsmCounterBytes = 256;
 
-// Bump-and-revalue legs sharing every normal: one request d_req (GBM step,
+// Bump-and-revalue legs sharing every normal: one request q (GBM step,
 // GBM terminal or Heston; xorshift, Sobol or counter-hash samples; any
-// technique) whose q.scen holds the legs' parameters; with NM =
+// technique) and its legs' parameters; tiles_done[0] and [1] are zero before and
+// after; with NM =
 // scenario_moments(technique), q.partials must hold [n_tiles][kMaxScen][NM]
 // doubles and q.moments [kMaxScen][NM]: sum p, sum p^2 (pair averages for
 // antithetic requests), then for control variates sum c, sum c^2, sum p c.
 constexpr int scenario_moments(int technique) { return technique == MPC_TECHNIQUE_CONTROL_VARIATE ? 5 : 2; }
-cudaError_t launch_scenarios(const DevReq* d_req, uint32_t n_tiles, uint32_t* d_counter, int family, int sampler,
-                             int technique, const DeviceTables& tabs, int grid, cudaStream_t stream);
+struct ScenarioLegs {
+  float f[kScenFields * kMaxScen];  // [field][leg]
+};
+cudaError_t launch_scenarios(const DevReq& q, const ScenarioLegs& legs, int family, int sampler, int technique,
+                             const DeviceTables& tabs, int grid, cudaStream_t stream);
 int scenario_max_blocks_per_sm(int family, int sampler, int technique);
 
-// Basket bump legs sharing every normal: one basket request d_req
+// Basket bump legs sharing every normal: one basket request q
 // (xorshift, Sobol or counter-hash samples); q.partials must hold
 // [n_tiles][kBasketScen][2] doubles and q.moments [kBasketScen][2].
-cudaError_t launch_basket_scenarios(const DevReq* d_req, uint32_t n_tiles, uint32_t* d_counter, int sampler,
-                                    const BasketScen& legs, const DeviceTables& tabs, int grid, cudaStream_t stream);
+cudaError_t launch_basket_scenarios(const DevReq& q, int sampler, const BasketScen& legs, const DeviceTables& tabs,
+                                    int grid, cudaStream_t stream);
 int basket_scenario_max_blocks_per_sm(int sampler);
 
 // Single-pass Greek estimators of the terminal-GBM European call

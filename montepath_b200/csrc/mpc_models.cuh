@@ -896,30 +896,53 @@ __device__ __forceinline__ void unit_merton(const DevReq& q, Src& src, double& p
   ctl = (double)(st * disc);
 }
 
-// Sums over n steps of a path's D normals per step.
+// Sums over n steps of a path's D normals per step.  FP32 samples are summed
+// in FP32 over four steps at a time and in FP64 from there on: a sum of
+// hundreds of normals grows to 10 or 20, where FP32 adds lose 5e-7 each (a
+// 154,595 x 290 basket of small price: 2.7e-6 off with FP32 sums).
 template <class Real, int D, class Src>
 __device__ __forceinline__ void sum_step_normals(Src& src, uint32_t n, Real zs[D]) {
+  double total[D];
 #pragma unroll
-  for (int a = 0; a < D; ++a) zs[a] = (Real)0;
+  for (int a = 0; a < D; ++a) total[a] = 0.0;
   uint32_t dim = 0, s = 0;
-  if constexpr (kPairSource<Src>) {
-    // two steps are D pairs whatever D's parity
-    for (; s + 2 <= n; s += 2) {
+  if constexpr (sizeof(Real) == 4) {
+    for (; s + 4 <= n; s += 4) {
+      float part[D];
 #pragma unroll
-      for (int p = 0; p < D; ++p) {
-        const float2 z = src.n32x2(dim + 2 * p);
-        zs[(2 * p) % D] += z.x;
-        zs[(2 * p + 1) % D] += z.y;
+      for (int a = 0; a < D; ++a) part[a] = 0.0f;
+      if constexpr (kPairSource<Src>) {
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {  // two steps are D pairs whatever D's parity
+#pragma unroll
+          for (int p = 0; p < D; ++p) {
+            const float2 z = src.n32x2(dim + 2 * p);
+            part[(2 * p) % D] += z.x;
+            part[(2 * p + 1) % D] += z.y;
+          }
+          dim += 2 * D;
+        }
+      } else {
+#pragma unroll 1
+        for (int h = 0; h < 4; ++h) {
+          src.at_step(dim, D);
+#pragma unroll
+          for (int a = 0; a < D; ++a) part[a] += normal<Real>(src, dim + a);
+          dim += D;
+        }
       }
-      dim += 2 * D;
+#pragma unroll
+      for (int a = 0; a < D; ++a) total[a] += (double)part[a];
     }
   }
   for (; s < n; ++s) {
     src.at_step(dim, D);
 #pragma unroll
-    for (int a = 0; a < D; ++a) zs[a] += normal<Real>(src, dim + a);
+    for (int a = 0; a < D; ++a) total[a] += (double)normal<Real>(src, dim + a);
     dim += D;
   }
+#pragma unroll
+  for (int a = 0; a < D; ++a) zs[a] = (Real)total[a];
 }
 
 // d-asset basket, terminal or stepwise (basket_terminal_payoff, cpu.rs:7616-7635),

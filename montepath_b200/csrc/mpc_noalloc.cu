@@ -172,8 +172,12 @@ extern "C" int mpc_price_fused_noalloc(const mpc_request_t* req, mpc_result_t* o
   if (e != cudaSuccess) return reject(MPC_E_CUDA, std::string("upload: ") + cudaGetErrorString(e));
   const int occ = std::max(1, mpc::fused_max_blocks_per_sm(p.family, p.sampler, 256));
   const int grid = int(std::min<uint64_t>(uint64_t(ds->sm_count) * occ, q.n_tiles));
-  e = mpc::launch_fused(&ds->scratch->req, ds->scratch->tiles, q.n_tiles, &ds->scratch->tile_counter, p.family,
-                        p.sampler, ds->tabs, std::max(grid, 1), 256, s);
+  mpc::FusedWork work{};
+  work.n_tiles = q.n_tiles;
+  work.counter = &ds->scratch->tile_counter;
+  work.reqs = &ds->scratch->req;
+  work.tiles = ds->scratch->tiles;
+  e = mpc::launch_fused(work, p.family, p.sampler, ds->tabs, std::max(grid, 1), 256, s);
   if (e != cudaSuccess) return reject(MPC_E_CUDA, std::string("launch: ") + cudaGetErrorString(e));
   double moments[MPC_MOMENTS];
   e = cudaMemcpyAsync(moments, ds->scratch->moments, sizeof(moments), cudaMemcpyDeviceToHost, s);

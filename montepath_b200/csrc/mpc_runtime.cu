@@ -100,7 +100,7 @@ static int within_budget(mpc_context* ctx, const char* name, uint64_t bytes) {
                   "', beyond the HBM budget of " + std::to_string(ctx->budget) + " bytes");
 }
 
-static int pinned_staging(mpc_context* ctx, size_t bytes, void** out) {
+int pinned_staging(mpc_context* ctx, size_t bytes, void** out) {
   if (ctx->pinned_bytes < bytes) {
     if (ctx->pinned) {
       cudaStreamSynchronize(ctx->stream);
@@ -723,21 +723,22 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
   }
   if (total_tiles > (1ull << 31)) return fail(ctx, MPC_E_UNSUPPORTED, "batch too large (tiles)");
   // device buffers
-  void *d_reqs, *d_tiles, *d_part, *d_mom, *d_done, *d_counter, *d_unit = nullptr;
+  void *d_reqs, *d_tiles, *d_part, *d_done, *d_counter, *d_inline, *d_unit = nullptr;
   size_t groups = 0;
   if ((st = scratch(ctx, "reqs", n * sizeof(DevReq), &d_reqs))) return st;
   if ((st = scratch(ctx, "tiles", total_tiles * sizeof(Tile), &d_tiles))) return st;
   if ((st = scratch(ctx, "partials", total_tiles * MPC_MOMENTS * sizeof(double), &d_part))) return st;
-  if ((st = scratch(ctx, "moments", n * MPC_MOMENTS * sizeof(double), &d_mom))) return st;
   if ((st = scratch(ctx, "done", n * sizeof(uint32_t), &d_done))) return st;
+  // list launches clear their cursors first, inline launches find and leave
+  // theirs zero (two words each): separate buffers
   if ((st = scratch(ctx, "counter", 64 * sizeof(uint32_t), &d_counter))) return st;
+  if ((st = scratch(ctx, "inline_counter", 2 * 64 * sizeof(uint32_t), &d_inline))) return st;
   if (per_unit_host) {  // the kernel writes every unit of request 0; the copy-out is clipped to the capacity
     if ((st = scratch(ctx, "per_unit", reqs[0]->q.n_units * sizeof(double), &d_unit))) return st;
   }
   for (size_t i = 0; i < n; ++i) {
     DevReq& q = reqs[i]->q;
     q.partials = static_cast<double*>(d_part) + size_t(tile_base[i]) * MPC_MOMENTS;
-    q.moments = static_cast<double*>(d_mom) + i * MPC_MOMENTS;
     q.tiles_done = static_cast<uint32_t*>(d_done) + i;
     q.per_unit = (per_unit_host && i == 0) ? static_cast<double*>(d_unit) : nullptr;
   }
@@ -767,15 +768,26 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
   }
   groups = gl.size();
   if (groups > 64) return fail(ctx, MPC_E_UNSUPPORTED, "too many sampler groups");
-  size_t desc_bytes = n * sizeof(DevReq);
-  size_t tile_bytes = total_tiles * sizeof(Tile);
-  size_t mom_bytes = n * MPC_MOMENTS * sizeof(double);
+  // The moments land in pinned memory, written by the kernels themselves.
+  // When no group has more than kFusedInline requests, the descriptors travel
+  // as kernel parameters and the call is the launches alone; else descriptors
+  // and tile lists are copied in first.  A 10,000-path terminal call: 51 us with
+  // two copies in, a counter fill and a copy out around the same kernel, 29 us.
+  bool inlined = true;
+  for (const Group& g : gl) inlined = inlined && g.members.size() <= kFusedInline;
+  const size_t mom_bytes = n * MPC_MOMENTS * sizeof(double);
+  const size_t desc_bytes = inlined ? 0 : n * sizeof(DevReq);
+  const size_t tile_bytes = inlined ? 0 : total_tiles * sizeof(Tile);
   void* pin = nullptr;
-  if ((st = pinned_staging(ctx, desc_bytes + tile_bytes + mom_bytes + 256, &pin))) return st;
-  uint8_t* hp = static_cast<uint8_t*>(pin);
-  for (size_t i = 0; i < n; ++i) std::memcpy(hp + i * sizeof(DevReq), &reqs[i]->q, sizeof(DevReq));
+  if ((st = pinned_staging(ctx, mom_bytes + desc_bytes + tile_bytes + 256, &pin))) return st;
+  double* hm = static_cast<double*>(pin);
+  uint8_t* hp = static_cast<uint8_t*>(pin) + ((mom_bytes + 255) & ~size_t(255));
   Tile* ht = reinterpret_cast<Tile*>(hp + desc_bytes);
-  std::vector<uint32_t> group_first(groups), group_count(groups);
+  for (size_t i = 0; i < n; ++i) {
+    reqs[i]->q.moments = hm + i * MPC_MOMENTS;
+    if (!inlined) std::memcpy(hp + i * sizeof(DevReq), &reqs[i]->q, sizeof(DevReq));
+  }
+  std::vector<FusedWork> work(groups);
   uint64_t cursor = 0;
   for (size_t g = 0; g < groups; ++g) {
     std::vector<size_t> order = gl[g].members;
@@ -783,23 +795,36 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
       return double(reqs[a]->q.normals_per_unit + reqs[a]->q.n_steps) * reqs[a]->q.tile_units >
              double(reqs[b]->q.normals_per_unit + reqs[b]->q.n_steps) * reqs[b]->q.tile_units;
     });
-    group_first[g] = uint32_t(cursor);
-    for (size_t i : order)
-      for (uint32_t t = 0; t < reqs[i]->q.n_tiles; ++t) ht[cursor++] = Tile{uint32_t(i), t};
-    group_count[g] = uint32_t(cursor - group_first[g]);
+    FusedWork& w = work[g];
+    w.counter = inlined ? static_cast<uint32_t*>(d_inline) + 2 * g : static_cast<uint32_t*>(d_counter) + g;
+    w.reqs = static_cast<const DevReq*>(d_reqs);
+    w.tiles = static_cast<const Tile*>(d_tiles) + cursor;
+    w.n_inline = inlined ? uint32_t(order.size()) : 0u;
+    for (size_t k = 0; k < order.size(); ++k) {
+      const DevReq& q = reqs[order[k]]->q;
+      if (inlined) {
+        w.first[k] = w.n_tiles;
+        w.inl[k] = q;
+      } else {
+        for (uint32_t t = 0; t < q.n_tiles; ++t) ht[cursor++] = Tile{uint32_t(order[k]), t};
+      }
+      w.n_tiles += q.n_tiles;
+    }
   }
-  double* hm = reinterpret_cast<double*>(hp + desc_bytes + tile_bytes);
   std::vector<uint64_t> grids(groups);
   for (size_t g = 0; g < groups; ++g) {
     int occ = std::max(1, fused_max_blocks_per_sm(gl[g].family, gl[g].sampler, int(gl[g].block)));
-    grids[g] = std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sm_count) * occ, group_count[g]));
+    grids[g] = std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(ctx->sm_count) * occ, work[g].n_tiles));
   }
-  // The sequence between the events: descriptors and tile list in, counters
-  // zeroed, one launch per group, moments out.
+  // The sequence between the events: descriptors and tile lists in and
+  // counters zeroed when they are not inline, one launch per group.
   auto enqueue = [&]() -> cudaError_t {
-    cudaError_t e = cudaMemcpyAsync(d_reqs, hp, desc_bytes, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, ht, tile_bytes, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_counter, 0, groups * sizeof(uint32_t), ctx->stream);
+    cudaError_t e = cudaSuccess;
+    if (!inlined) {
+      e = cudaMemcpyAsync(d_reqs, hp, desc_bytes, cudaMemcpyHostToDevice, ctx->stream);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, ht, tile_bytes, cudaMemcpyHostToDevice, ctx->stream);
+      if (e == cudaSuccess) e = cudaMemsetAsync(d_counter, 0, groups * sizeof(uint32_t), ctx->stream);
+    }
     if (e == cudaSuccess && groups > 1) e = cudaEventRecord(ctx->ev_fork, ctx->stream);
     bool used[mpc_context::kSideStreams] = {};
     for (size_t g = 0; g < groups && e == cudaSuccess; ++g) {
@@ -813,9 +838,7 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
           if (e != cudaSuccess) break;
         }
       }
-      e = launch_fused(static_cast<DevReq*>(d_reqs), static_cast<Tile*>(d_tiles) + group_first[g], group_count[g],
-                       static_cast<uint32_t*>(d_counter) + g, gl[g].family, gl[g].sampler, ctx->tabs, int(grids[g]),
-                       int(gl[g].block), st);
+      e = launch_fused(work[g], gl[g].family, gl[g].sampler, ctx->tabs, int(grids[g]), int(gl[g].block), st);
     }
     for (int k = 0; k < mpc_context::kSideStreams; ++k) {  // join every forked stream, also after an error
       if (!used[k]) continue;
@@ -823,19 +846,21 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
       const cudaError_t ew = ej == cudaSuccess ? cudaStreamWaitEvent(ctx->stream, ctx->ev_join[k], 0) : ej;
       if (e == cudaSuccess) e = ew;
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hm, d_mom, mom_bytes, cudaMemcpyDeviceToHost, ctx->stream);
     return e;
   };
   // everything the sequence bakes in: addresses, sizes, launch shapes
-  std::vector<uint64_t> key = {uint64_t(uintptr_t(hp)), uint64_t(uintptr_t(d_reqs)), uint64_t(uintptr_t(d_tiles)),
-                               uint64_t(uintptr_t(d_counter)), uint64_t(uintptr_t(d_mom)),
-                               uint64_t(uintptr_t(ctx->tabs.sobol)), desc_bytes, tile_bytes, mom_bytes, groups};
-  for (size_t g = 0; g < groups; ++g)
-    key.insert(key.end(), {uint64_t(int64_t(gl[g].family)), uint64_t(gl[g].sampler), uint64_t(gl[g].block), grids[g],
-                           group_first[g], group_count[g]});
+  // (inline descriptors are part of the launches, which then need no graph)
+  std::vector<uint64_t> key;
+  if (!inlined) {
+    key = {uint64_t(uintptr_t(hp)), uint64_t(uintptr_t(d_reqs)), uint64_t(uintptr_t(d_tiles)),
+           uint64_t(uintptr_t(d_counter)), uint64_t(uintptr_t(ctx->tabs.sobol)), desc_bytes, tile_bytes, groups};
+    for (size_t g = 0; g < groups; ++g)
+      key.insert(key.end(), {uint64_t(int64_t(gl[g].family)), uint64_t(gl[g].sampler), uint64_t(gl[g].block), grids[g],
+                             uint64_t(uintptr_t(work[g].tiles)), work[g].n_tiles});
+  }
   uint64_t launches_before = kernel_launch_count();
-  bool replay = ctx->graph_exec && key == ctx->graph_key;
-  if (!replay && key == ctx->last_batch_key) {  // second time in a row: capture (host only), then replay
+  bool replay = !inlined && ctx->graph_exec && key == ctx->graph_key;
+  if (!inlined && !replay && key == ctx->last_batch_key) {  // second time in a row: capture (host only), then replay
     if (ctx->graph_exec) {
       cudaGraphExecDestroy(ctx->graph_exec);
       ctx->graph_exec = nullptr;
@@ -870,14 +895,14 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
     const cudaError_t e = enqueue();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "fused pricing batch");
   }
-  ctx->last_batch_key = key;
+  if (!inlined) ctx->last_batch_key = key;
   MPC_CUDA(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
   MPC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
   ctx->last_ms = ms;
   ctx->last_launches = kernel_launch_count() - launches_before;
-  ctx->last_h2d = desc_bytes + tile_bytes;
+  ctx->last_h2d = inlined ? n * sizeof(DevReq) : desc_bytes + tile_bytes;  // inline: as kernel parameters
   ctx->last_d2h = mom_bytes;
   for (size_t i = 0; i < n; ++i) {
     summarize_moments(*reqs[i], hm + i * MPC_MOMENTS, outs[i]);
@@ -950,7 +975,7 @@ static int run_plain(mpc_context* ctx, Prepared* p, mpc_result_t* out, double* p
   cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
   ctx->last_ms = ms;
   ctx->last_launches = kernel_launch_count() - launches_before;
-  ctx->last_h2d = 0;
+  ctx->last_h2d = sizeof(DevReq);  // as a kernel parameter
   ctx->last_d2h = MPC_MOMENTS * sizeof(double);
   summarize_moments(*p, hm, out);
   out->path_steps = p->path_steps;
@@ -1029,7 +1054,7 @@ static int run_merton_stream(mpc_context* ctx, Prepared* p, mpc_result_t* out, d
   cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
   ctx->last_ms = ms;
   ctx->last_launches = kernel_launch_count() - launches_before;
-  ctx->last_h2d = 0;
+  ctx->last_h2d = sizeof(MertonStreamArgs);  // as kernel parameters
   ctx->last_d2h = 3 * sizeof(double);
   summarize_moments(*p, hm, out);
   out->path_steps = p->path_steps;

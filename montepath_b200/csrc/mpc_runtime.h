@@ -109,6 +109,8 @@ int fail(mpc_context* ctx, int status, const std::string& msg);
 int cuda_fail(mpc_context* ctx, cudaError_t err, const char* what);
 // Returns a device buffer of at least `bytes` for `name`, growing it under the budget.
 int scratch(mpc_context* ctx, const std::string& name, size_t bytes, void** out);
+// Pinned host memory of at least `bytes` (mapped: kernels write results there), one area per context.
+int pinned_staging(mpc_context* ctx, size_t bytes, void** out);
 int validate(const mpc_request_t& r, std::string* msg);
 int prepare(mpc_context* ctx, const mpc_request_t& r, Prepared* p, std::string* msg);
 uint64_t estimate_bytes(const mpc_request_t& r);

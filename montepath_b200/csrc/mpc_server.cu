@@ -352,8 +352,12 @@ int run_wave(mpc_server* s, std::unique_lock<std::mutex>& lk) {
       int fam = family_of[kv.first];
       int occ = std::max(1, fused_max_blocks_per_sm(fam, kv.first, 256));
       uint64_t grid = std::min<uint64_t>(uint64_t(s->ctx->sm_count) * occ, kv.second.size());
-      cudaError_t e = launch_fused(s->d_slots, s->d_tiles + first, uint32_t(kv.second.size()), s->d_counter + g_idx,
-                                   fam, kv.first, s->ctx->tabs, int(std::max<uint64_t>(grid, 1)), 256, s->stream);
+      FusedWork work{};
+      work.n_tiles = uint32_t(kv.second.size());
+      work.counter = s->d_counter + g_idx;
+      work.reqs = s->d_slots;
+      work.tiles = s->d_tiles + first;
+      cudaError_t e = launch_fused(work, fam, kv.first, s->ctx->tabs, int(std::max<uint64_t>(grid, 1)), 256, s->stream);
       if (e != cudaSuccess) status = MPC_E_CUDA;
       first += kv.second.size();
       ++g_idx;

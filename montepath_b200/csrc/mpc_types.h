@@ -113,8 +113,7 @@ struct alignas(16) DevReq {
   const uint32_t* bridge_events;  // [(2 n_steps - 1 + 31) / 32]
   double bridge_sqrt_t, bridge_inv_sqrt_dt;
   uint32_t bridge;                // 1: normals come through the bridge
-  uint32_t n_scen;                // scenario kernel: legs in `scen` (0 elsewhere)
-  const float* scen;              // scenario kernel: [kScenFields][kMaxScen] leg parameters
+  uint32_t n_scen;                // scenario kernel: legs (0 elsewhere)
   // samplers
   const uint32_t* halton_primes;
   const double* halton_shifts;

@@ -41,3 +41,21 @@ def test_baskets_by_pairs(backend, assets, n_steps, sampling, technique):
     check(backend, "basket_call", dict(method="stepwise", n_steps=n_steps, n_paths=2001, seed=6, sampling=sampling,
                                        technique=technique, spots=[90.0 + 4.0 * i for i in range(assets)],
                                        sigmas=[0.15 + 0.03 * i for i in range(assets)], corr=corr))
+
+
+@pytest.mark.parametrize("members", [1, 4, 5])
+def test_inline_and_listed_groups(backend, members):
+    """Groups of up to four requests travel as launch parameters, larger ones
+    through a tile list: the same prices either way, alternating, with more
+    tiles than resident blocks and with a single one."""
+
+    reqs = [make_request("european_call", dict(method="stepwise", n_steps=3 + i, seed=i, sampling="counter_hash",
+                                               n_paths=(400_001 if i % 2 else 77)))
+            for i in range(members)]
+    reqs.append(make_request("basket_call", dict(n_paths=5000, seed=1)))
+    alone = [backend.price(r) for r in reqs]
+    for _ in range(3):
+        for a, b in zip(alone, backend.price_batch(reqs)):
+            assert (a.price, a.stderr, a.n_samples) == (b.price, b.stderr, b.n_samples)
+        for r, a in zip(reqs, alone):
+            assert backend.price(r).price == a.price
