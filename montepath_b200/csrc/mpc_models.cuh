@@ -172,48 +172,48 @@ struct Source<SMP_SOBOL> {
 template <>
 struct Source<SMP_HALTON> {
   uint64_t index;
-  const uint32_t* primes;
-  const double* shifts;
+  const HaltonDim* dims;
+  const double* weights;
   template <bool FP64>
   __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx&, uint64_t u) {
     index = u + 1;
-    primes = q.halton_primes;
-    shifts = q.halton_shifts;
+    dims = q.halton;
+    weights = q.halton_weights;
   }
   __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ double u64(uint32_t d) { return halton_shifted(index, __ldg(primes + d), __ldg(shifts + d)); }
+  __device__ __forceinline__ double u64(uint32_t d) { return halton_f64(index, dims + d, weights); }
   __device__ __forceinline__ double n64(uint32_t d) { return icdf_f64(u64(d)); }
+  __device__ __forceinline__ float u32(uint32_t d) { return (float)halton_f32(index, dims + d); }
   __device__ __forceinline__ float n32(uint32_t d) {
-    float u = fminf(fmaxf((float)u64(d), 5.9604645e-08f), 0.99999994f);
+    float u = fminf(fmaxf(u32(d), 5.9604645e-08f), 0.99999994f);
     return normcdfinvf(u);
   }
-  __device__ __forceinline__ float u32(uint32_t d) { return (float)u64(d); }
 };
 
 template <>
 struct Source<SMP_LHS> {
-  uint64_t point, n_paths;
+  uint64_t point, mixed, n_paths;
+  double inv_n;  // FP32 samples scale by it; FP64 ones divide, as the reference does
   const LhsDim* dims;
   template <bool FP64>
   __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx&, uint64_t u) {
     point = u;
+    mixed = u * 0xBF58476D1CE4E5B9ull;
     n_paths = q.n_paths;
+    inv_n = 1.0 / (double)n_paths;
     dims = q.lhs;
   }
   __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
   __device__ __forceinline__ double u64(uint32_t d) {
-    LhsDim ld;
-    ld.multiplier = __ldg(&dims[d].multiplier);
-    ld.offset = __ldg(&dims[d].offset);
-    ld.jitter_seed = __ldg(&dims[d].jitter_seed);
-    return lhs_uniform(ld, point, n_paths);
+    const double u = lhs_place(dims + d, point, mixed, n_paths) / (double)n_paths;
+    return fmin(fmax(u, 2.2250738585072014e-308), 1.0 - 2.220446049250313e-16);
   }
   __device__ __forceinline__ double n64(uint32_t d) { return icdf_f64(u64(d)); }
+  __device__ __forceinline__ float u32(uint32_t d) { return (float)(lhs_place(dims + d, point, mixed, n_paths) * inv_n); }
   __device__ __forceinline__ float n32(uint32_t d) {
-    float u = fminf(fmaxf((float)u64(d), 5.9604645e-08f), 0.99999994f);
+    float u = fminf(fmaxf(u32(d), 5.9604645e-08f), 0.99999994f);
     return normcdfinvf(u);
   }
-  __device__ __forceinline__ float u32(uint32_t d) { return (float)u64(d); }
 };
 
 template <>
@@ -564,62 +564,71 @@ __device__ __forceinline__ uint32_t poisson_tail(double u, double mean, double p
 // fill_step_normals_from_inputs (cpu.rs:5964-5981) as a streaming walk: the
 // reference fills w[0..n] op by op and then differences it; here the same
 // ops run in the same (depth-first) order, but only the right endpoints still
-// needed stay on a small stack, and each leaf yields the next step's
-// increment (w[s] - w[s-1]) / sqrt(dt) at once.  Input dimensions are drawn in
-// increasing order (0 = W(T), then one per op), every thread of a request
-// runs the same event sequence, so block-synchronous sources stay in lockstep.
-// FP64 keeps the reference's two-rounding products and left-to-right sums.
-template <class Real>
+// needed stay on a small stack (the nearest one in a register), and each step
+// yields its increment (w[s] - w[s-1]) / sqrt(dt) at once.  Input dimensions are
+// drawn in increasing order (0 = W(T), then one per op), a quad of them at a
+// time; every thread of a request runs the same sequence, so the staged Sobol
+// source stays in lockstep.  FP64 keeps the reference's two-rounding products
+// and left-to-right sums.  The weights come in the path's precision (one
+// 16-byte load an op), the op counts by step instead of an event bit each, and
+// the samples by quads: 123 instructions a step in FP32, which alone is bound by
+// latency (60 us for 100,000 x 64, as before) and beside other groups by issue.
+template <class Real, class Src>
 struct BridgeWalk {
+  static_assert(kQuadSource<Src>, "bridge paths are drawn from scrambled Sobol");
   Real stack[kBridgeDepth];
-  Real w_left;
-  uint32_t sp, ev, op, dim;
+  Real w_left, top;
+  Real z0, z1, z2, z3;  // the current quad's normals
+  uint32_t sp, op, dim;
 
-  __device__ __forceinline__ static Real mid(Real lw, Real wl, Real rw, Real wr, Real sd, Real z) {
-    if constexpr (sizeof(Real) == 8)
-      return __dadd_rn(__dadd_rn(__dmul_rn(lw, wl), __dmul_rn(rw, wr)), __dmul_rn(sd, z));
-    else
-      return lw * wl + rw * wr + sd * z;
-  }
-  template <class Src>
-  __device__ __forceinline__ void begin(const DevReq& q, Src& src) {
-    src.at_step(0, 1);
-    const Real z0 = normal<Real>(src, 0);
-    if constexpr (sizeof(Real) == 8)
-      stack[0] = __dmul_rn(q.bridge_sqrt_t, z0);
-    else
-      stack[0] = (Real)q.bridge_sqrt_t * z0;
-    sp = 1;
-    w_left = (Real)0;
-    ev = 0;
-    op = 0;
-    dim = 1;
-  }
-  // The increment of the next step (the host checked the program: it ends
-  // every op run with a leaf and never needs more than kBridgeDepth values).
-  template <class Src>
-  __device__ __forceinline__ Real next(const DevReq& q, Src& src) {
-    for (;;) {
-      const uint32_t is_op = (__ldg(q.bridge_events + (ev >> 5)) >> (ev & 31)) & 1u;
-      ++ev;
-      if (!is_op) break;
-      const double* o = q.bridge_ops + 3 * op;
-      ++op;
-      src.at_step(dim, 1);
-      const Real z = normal<Real>(src, dim);
-      ++dim;
-      const Real wr = stack[sp - 1];
-      stack[sp] = mid((Real)__ldg(o), w_left, (Real)__ldg(o + 1), wr, (Real)__ldg(o + 2), z);
-      ++sp;
+  __device__ __forceinline__ Real draw(Src& src) {
+    const uint32_t k = dim & 3u;
+    if (k == 0) {
+      src.at_step(dim, 4);
+      src.quad_load(dim);
+      const auto a = src.template take_n2<0, 1>(dim), b = src.template take_n2<2, 3>(dim);
+      z0 = a.x;
+      z1 = a.y;
+      z2 = b.x;
+      z3 = b.y;
     }
-    --sp;
-    const Real wr = stack[sp];
+    ++dim;
+    return k & 2u ? (k & 1u ? z3 : z2) : (k & 1u ? z1 : z0);
+  }
+  __device__ __forceinline__ void begin(const DevReq& q, Src& src) {
+    dim = 0;
+    const Real z = draw(src);
+    if constexpr (sizeof(Real) == 8)
+      top = __dmul_rn(q.bridge_sqrt_t, z);
+    else
+      top = (Real)q.bridge_sqrt_t * z;
+    sp = 0;
+    w_left = (Real)0;
+    op = 0;
+  }
+  // The increment of step s (the host checked the program: it never needs
+  // more than kBridgeDepth values).
+  __device__ __forceinline__ Real next(const DevReq& q, Src& src, uint32_t s) {
+    for (uint32_t left = __ldg(q.bridge_counts + s); left > 0; --left, ++op) {
+      const Real z = draw(src);
+      stack[sp++] = top;
+      if constexpr (sizeof(Real) == 8) {
+        const double2* o = static_cast<const double2*>(q.bridge_ops) + 2 * op;
+        const double2 w = __ldg(o);
+        const double sd = __ldg(reinterpret_cast<const double*>(o + 1));
+        top = __dadd_rn(__dadd_rn(__dmul_rn(w.x, w_left), __dmul_rn(w.y, top)), __dmul_rn(sd, z));
+      } else {
+        const float4 o = __ldg(static_cast<const float4*>(q.bridge_ops) + op);
+        top = o.x * w_left + o.y * top + o.z * z;
+      }
+    }
     Real inc;
     if constexpr (sizeof(Real) == 8)
-      inc = __dmul_rn(__dsub_rn(wr, w_left), q.bridge_inv_sqrt_dt);
+      inc = __dmul_rn(__dsub_rn(top, w_left), q.bridge_inv_sqrt_dt);
     else
-      inc = (wr - w_left) * (Real)q.bridge_inv_sqrt_dt;
-    w_left = wr;
+      inc = (top - w_left) * (Real)q.bridge_inv_sqrt_dt;
+    w_left = top;
+    if (sp > 0) top = stack[--sp];
     return inc;
   }
 };
@@ -667,9 +676,9 @@ __device__ __forceinline__ void unit_gbm_step(const DevReq& q, Src& src, double&
   };
   uint32_t s = 0;
   if constexpr (BRIDGE) {  // increments from the Brownian bridge over the inputs
-    BridgeWalk<Real> bw;
+    BridgeWalk<Real, Src> bw;
     bw.begin(q, src);
-    for (; s < n; ++s) advance(bw.next(q, src));
+    for (; s < n; ++s) advance(bw.next(q, src, s));
   } else if constexpr (kQuadSource<Src>) {
     for (; s + 4 <= n; s += 4) {  // four steps per quad of dimensions
       src.at_step(s, 4);

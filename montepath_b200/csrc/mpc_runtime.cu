@@ -100,23 +100,27 @@ static int within_budget(mpc_context* ctx, const char* name, uint64_t bytes) {
                   "', beyond the HBM budget of " + std::to_string(ctx->budget) + " bytes");
 }
 
-int pinned_staging(mpc_context* ctx, size_t bytes, void** out) {
-  if (ctx->pinned_bytes < bytes) {
-    if (ctx->pinned) {
+static int grow_pinned(mpc_context* ctx, void** area, size_t* held, size_t bytes, void** out) {
+  if (*held < bytes) {
+    if (*area) {
       cudaStreamSynchronize(ctx->stream);
-      cudaFreeHost(ctx->pinned);
+      cudaFreeHost(*area);
     }
-    size_t grow = std::max(bytes, ctx->pinned_bytes * 2);
-    cudaError_t err = cudaHostAlloc(&ctx->pinned, grow, cudaHostAllocDefault);
+    size_t grow = std::max(bytes, *held * 2);
+    cudaError_t err = cudaHostAlloc(area, grow, cudaHostAllocDefault);
     if (err != cudaSuccess) {
-      ctx->pinned = nullptr;
-      ctx->pinned_bytes = 0;
+      *area = nullptr;
+      *held = 0;
       return cuda_fail(ctx, err, "cudaHostAlloc");
     }
-    ctx->pinned_bytes = grow;
+    *held = grow;
   }
-  *out = ctx->pinned;
+  *out = *area;
   return MPC_OK;
+}
+
+int pinned_staging(mpc_context* ctx, size_t bytes, void** out) {
+  return grow_pinned(ctx, &ctx->pinned, &ctx->pinned_bytes, bytes, out);
 }
 
 // ------------------------------------------------------------ validation ---
@@ -345,23 +349,24 @@ static int sampler_of(int sampling) {
   }
 }
 
-// BrownianBridgePlan::new (cpu.rs:5923-5962) flattened into the event
-// program the device walks: the reference's interval stack is replayed and
-// every pop becomes an event -- an op (midpoint of an interval longer than
-// one step, consuming the next input dimension) or a leaf (one step).  Ops
-// carry the reference's weights and stddev, computed the same way.  Returns
-// false if the walk would need a deeper stack than the device holds.
+// BrownianBridgePlan::new (cpu.rs:5923-5962) flattened into the program the
+// device walks: the reference's interval stack is replayed; every pop is an op
+// (a midpoint of an interval longer than one step, consuming the next input
+// dimension) or a step, and a step records how many ops came before it since
+// the last one.  Ops carry the reference's weights and stddev, computed the same
+// way.  Returns false if the walk would need a deeper stack than the device holds.
 static bool build_bridge_program(Prepared* p, uint32_t n, double maturity) {
   const double dt = maturity / double(n);
   p->bridge_ops.clear();
-  p->bridge_events.assign((2ull * n - 1 + 31) / 32, 0u);
+  p->bridge_counts.clear();
   std::vector<std::pair<uint32_t, uint32_t>> intervals{{0u, n}};
-  uint32_t event = 0, depth = 1, max_depth = 1;  // depth: values on the device stack (starts with W(T))
+  uint32_t ops = 0, depth = 1, max_depth = 1;  // depth: values on the device stack (starts with W(T))
   while (!intervals.empty()) {
     const auto [left, right] = intervals.back();
     intervals.pop_back();
-    if (right <= left + 1) {  // leaf: pops one value
-      ++event;
+    if (right <= left + 1) {  // a step: pops one value
+      p->bridge_counts.push_back(uint8_t(ops));
+      ops = 0;
       --depth;
       continue;
     }
@@ -371,15 +376,15 @@ static bool build_bridge_program(Prepared* p, uint32_t n, double maturity) {
     p->bridge_ops.push_back((t_right - t_mid) / denom);
     p->bridge_ops.push_back((t_mid - t_left) / denom);
     p->bridge_ops.push_back(std::sqrt((t_mid - t_left) * (t_right - t_mid) / denom));
-    p->bridge_events[event >> 5] |= 1u << (event & 31);
-    ++event;
+    p->bridge_ops.push_back(0.0);
+    ++ops;
     max_depth = std::max(max_depth, ++depth);  // op: pushes the midpoint
     intervals.push_back({mid, right});
     intervals.push_back({left, mid});
   }
   p->q.bridge_sqrt_t = std::sqrt(maturity);
   p->q.bridge_inv_sqrt_dt = 1.0 / std::sqrt(dt);
-  return event == 2 * n - 1 && depth == 0 && max_depth <= kBridgeDepth && p->bridge_ops.size() == 3ull * (n - 1);
+  return p->bridge_counts.size() == n && depth == 0 && max_depth <= kBridgeDepth && p->bridge_ops.size() == 4ull * (n - 1);
 }
 
 static std::vector<uint32_t> first_primes(size_t n) {
@@ -419,10 +424,31 @@ static uint64_t gcd64(uint64_t a, uint64_t b) {
 static void build_sampler_tables(Prepared* p, uint64_t seed, uint64_t n_paths, uint64_t dims) {
   if (p->sampler == SMP_HALTON) {
     size_t count = std::max<size_t>(dims, 2);
-    p->halton_primes = first_primes(count);
-    p->halton_shifts.resize(count);
-    for (size_t d = 0; d < count; ++d)
-      p->halton_shifts[d] = open01_u64(splitmix64(seed + uint64_t(d) * 0x9E3779B97F4A7C15ull));
+    const std::vector<uint32_t> primes = first_primes(count);
+    p->halton.resize(count);
+    for (size_t d = 0; d < count; ++d) {
+      HaltonDim& h = p->halton[d];
+      h = HaltonDim{};
+      h.base = primes[d];
+      h.offset = open01_u64(splitmix64(seed + uint64_t(d) * 0x9E3779B97F4A7C15ull));
+      if (n_paths >= 0x7FFFFFFFull) continue;  // indices up to n_paths: the general loop from 2^31 on
+      // n / base = (n m) >> (31 + L) for n < 2^31 with L = ceil(log2 base), m = ceil(2^(31 + L) / base)
+      uint32_t log = 0;
+      while ((1ull << log) < h.base) ++log;
+      h.shift = uint8_t(log - 1);
+      h.magic = uint32_t(((1ull << (31 + log)) + h.base - 1) / h.base);
+      h.weights_at = uint32_t(p->halton_weights.size());
+      uint64_t power = 1;
+      double f = 1.0 / double(h.base);
+      while (power <= n_paths) {
+        power *= h.base;
+        ++h.digits;
+        p->halton_weights.push_back(f);
+        f /= double(h.base);
+      }
+      h.wide = power >> 32 ? 1 : 0;
+      h.inv = 1.0 / double(power);
+    }
   } else if (p->sampler == SMP_LHS) {
     size_t count = std::max<size_t>(dims, 1);
     p->lhs.resize(count);
@@ -440,6 +466,8 @@ static void build_sampler_tables(Prepared* p, uint64_t seed, uint64_t n_paths, u
       p->lhs[d].multiplier = c;
       p->lhs[d].offset = n_paths == 0 ? 0 : splitmix64(mixed ^ 0xA24BAED4963EE407ull) % n_paths;
       p->lhs[d].jitter_seed = splitmix64(mixed ^ 0x9FB21C651E98DF25ull);
+      p->lhs[d].small = modulus < 0x80000000ull && (c < modulus || modulus == 1) ? 1 : 0;
+      p->lhs[d].shoup = p->lhs[d].small && modulus > 1 ? uint32_t((c << 32) / modulus) : 0u;
     }
   }
 }
@@ -660,45 +688,55 @@ void summarize_moments(const Prepared& p, const double* m, mpc_result_t* out) {
   summarize(n, m[1], m[2], &out->price, &out->stderr);
 }
 
-// Uploads the sampler tables of `reqs` into one aux buffer and points the descriptors at them.
+// Uploads the sampler tables of `reqs` into one aux buffer and points the
+// descriptors at them.  The copy is asynchronous from a pinned area of its own
+// (every call that uploads also waits for its stream before it returns).
 static int upload_aux(mpc_context* ctx, std::vector<Prepared*>& reqs) {
   size_t bytes = 0;
-  for (Prepared* p : reqs) {
-    bytes += p->halton_primes.size() * 4 + 16;
-    bytes += p->halton_shifts.size() * 8 + 16;
-    bytes += p->lhs.size() * sizeof(LhsDim) + 16;
-    bytes += p->bridge_ops.size() * 8 + p->bridge_events.size() * 4 + 32;
-  }
   bool any = false;  // per-request tables to place
-  for (Prepared* p : reqs) any = any || !p->halton_primes.empty() || !p->lhs.empty() || p->q.bridge;
+  for (Prepared* p : reqs) {
+    bytes += p->halton.size() * sizeof(HaltonDim) + p->halton_weights.size() * 8 + 32;
+    bytes += p->lhs.size() * sizeof(LhsDim) + 16;
+    bytes += p->bridge_ops.size() * 8 + p->bridge_counts.size() + 32;
+    any = any || !p->halton.empty() || !p->lhs.empty() || p->q.bridge;
+  }
   if (!any) return MPC_OK;
-  void* d_aux = nullptr;
+  void *d_aux = nullptr, *pin = nullptr;
   int st = scratch(ctx, "aux", bytes, &d_aux);
+  if (st == MPC_OK) st = grow_pinned(ctx, &ctx->pinned_aux, &ctx->pinned_aux_bytes, bytes, &pin);
   if (st != MPC_OK) return st;
-  std::vector<uint8_t> host(bytes);
+  uint8_t* host = static_cast<uint8_t*>(pin);
   size_t off = 0;
+  auto reserve = [&](size_t n) {
+    const size_t at = (off + 15) & ~size_t(15);
+    off = at + n;
+    return at;
+  };
   auto place = [&](const void* src, size_t n) -> void* {
-    off = (off + 15) & ~size_t(15);
-    std::memcpy(host.data() + off, src, n);
-    void* dev = static_cast<uint8_t*>(d_aux) + off;
-    off += n;
-    return dev;
+    const size_t at = reserve(n);
+    std::memcpy(host + at, src, n);
+    return static_cast<uint8_t*>(d_aux) + at;
   };
   for (Prepared* p : reqs) {
-    if (!p->halton_primes.empty()) {
-      p->q.halton_primes = static_cast<const uint32_t*>(place(p->halton_primes.data(), p->halton_primes.size() * 4));
-      p->q.halton_shifts = static_cast<const double*>(place(p->halton_shifts.data(), p->halton_shifts.size() * 8));
+    if (!p->halton.empty()) {
+      p->q.halton = static_cast<const HaltonDim*>(place(p->halton.data(), p->halton.size() * sizeof(HaltonDim)));
+      p->q.halton_weights =
+          static_cast<const double*>(place(p->halton_weights.data(), p->halton_weights.size() * sizeof(double)));
     }
     if (!p->lhs.empty()) p->q.lhs = static_cast<const LhsDim*>(place(p->lhs.data(), p->lhs.size() * sizeof(LhsDim)));
-    if (p->q.bridge) {  // a one-step program has a leaf event and no op
-      if (!p->bridge_ops.empty())
-        p->q.bridge_ops = static_cast<const double*>(place(p->bridge_ops.data(), p->bridge_ops.size() * 8));
-      p->q.bridge_events =
-          static_cast<const uint32_t*>(place(p->bridge_events.data(), p->bridge_events.size() * 4));
+    if (p->q.bridge) {  // a one-step program has no op
+      if (p->plain) {
+        p->q.bridge_ops = place(p->bridge_ops.data(), p->bridge_ops.size() * 8);
+      } else {
+        const size_t at = reserve(p->bridge_ops.size() * 4);
+        float* out = reinterpret_cast<float*>(host + at);
+        for (size_t i = 0; i < p->bridge_ops.size(); ++i) out[i] = float(p->bridge_ops[i]);
+        p->q.bridge_ops = static_cast<uint8_t*>(d_aux) + at;
+      }
+      p->q.bridge_counts = static_cast<const uint8_t*>(place(p->bridge_counts.data(), p->bridge_counts.size()));
     }
   }
-  MPC_CUDA(ctx, cudaMemcpyAsync(d_aux, host.data(), off, cudaMemcpyHostToDevice, ctx->stream));
-  MPC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  MPC_CUDA(ctx, cudaMemcpyAsync(d_aux, host, off, cudaMemcpyHostToDevice, ctx->stream));
   return MPC_OK;
 }
 
@@ -2337,6 +2375,7 @@ int mpc_destroy(mpc_context_t* ctx) {
   if (ctx->d_jump) cudaFree(ctx->d_jump);
   if (ctx->d_icdf_tail) cudaFree(ctx->d_icdf_tail);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
+  if (ctx->pinned_aux) cudaFreeHost(ctx->pinned_aux);
   if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
   if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);

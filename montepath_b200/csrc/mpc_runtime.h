@@ -39,11 +39,11 @@ struct Prepared {
   uint32_t ppt_hint = 0;  // request's paths_per_thread (0: autotuner)
   uint32_t block_hint = 0;  // request's block_size (0: autotuner)
   double cv_expectation = 0.0;
-  std::vector<uint32_t> halton_primes;
-  std::vector<double> halton_shifts;
+  std::vector<HaltonDim> halton;
+  std::vector<double> halton_weights;
   std::vector<LhsDim> lhs;
-  std::vector<double> bridge_ops;
-  std::vector<uint32_t> bridge_events;
+  std::vector<double> bridge_ops;       // [n_steps - 1][4]
+  std::vector<uint8_t> bridge_counts;   // [n_steps]
   uint64_t path_steps = 0;
 };
 
@@ -84,6 +84,8 @@ struct mpc_context {
   std::map<std::string, mpc::DevBuf> bufs;  // named scratch buffers
   void* pinned = nullptr;                   // pinned staging for descriptors and results
   size_t pinned_bytes = 0;
+  void* pinned_aux = nullptr;               // pinned staging for sampler tables
+  size_t pinned_aux_bytes = 0;
   mpc::Autotuner tuner;
   // CUDA graph of the fused batch sequence (copies in, launches, copy out):
   // captured when the same batch shape comes twice in a row, replayed while

@@ -877,7 +877,7 @@ int mpc_submit(mpc_server_t* s, const mpc_request_t* req, uint64_t* ticket) {
       req->workload != MPC_WORKLOAD_BERMUDAN_PUT) {
     st = prepare(s->ctx, *req, &t.prep, &msg);
     if (st == MPC_OK && !t.prep.plain && s->opt.mode != 1) {
-      if (!t.prep.halton_primes.empty() || !t.prep.lhs.empty() || t.prep.q.bridge || merton_stream_request(*req))
+      if (!t.prep.halton.empty() || !t.prep.lhs.empty() || t.prep.q.bridge || merton_stream_request(*req))
         t.prep.plain = true;  // per-request tables or the Merton stream replay: their own launches
       else if (!shape_for_slot(s, &t.prep))
         t.prep.plain = true;  // too many tiles for a slot: priced as its own batch

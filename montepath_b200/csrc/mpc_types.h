@@ -68,8 +68,24 @@ enum Sampler : int32_t {
   SMP_COUNTER = 5,
 };
 
-struct LhsDim {
+// One dimension of a Latin hypercube: stratum (multiplier point + offset) mod
+// n.  `shoup` = floor(multiplier 2^32 / n) gives that remainder without a
+// division for n < 2^31 (`small`).
+struct alignas(16) LhsDim {
   uint64_t multiplier, offset, jitter_seed;
+  uint32_t shoup, small;
+};
+// One dimension of a randomized Halton sequence of at most n points: indices
+// have up to `digits` base-`base` digits (base^digits > n); index / base is
+// (index * magic) >> (32 + shift) for index < 2^31.  FP32 samples take the
+// digits' reversed number times inv = base^-digits; FP64 ones sum digit times
+// the reference's own quotients 1 / base, (1 / base) / base, ..., tabulated from
+// weights_at on.  digits 0: the general loop.
+struct alignas(16) HaltonDim {
+  uint32_t base, magic;
+  uint8_t shift, digits, wide, pad;  // wide: base^digits needs 64 bits
+  uint32_t weights_at;
+  double inv, offset;                   // offset: the random shift
 };
 
 // Everything a tile needs to simulate units of one request.  Built on the
@@ -105,18 +121,17 @@ struct alignas(16) DevReq {
   uint32_t level, refinement;
   uint64_t coarse_steps;
   double f_drift, f_vol, c_drift, c_vol, inv_sqrt_m, inv_fine, inv_coarse;
-  // Brownian-bridge path construction (GBM stepwise with bridge Sobol): a
-  // program of 2 n_steps - 1 events in the reference's depth-first order;
-  // event e is an op (a midpoint, weights and stddev in bridge_ops) when bit
-  // e of bridge_events is set, else a leaf (one step increment).
-  const double* bridge_ops;       // [n_steps - 1][3]: left weight, right weight, stddev
-  const uint32_t* bridge_events;  // [(2 n_steps - 1 + 31) / 32]
+  // Brownian-bridge path construction (GBM stepwise with bridge Sobol), in the
+  // reference's depth-first order: step s is preceded by bridge_counts[s] ops
+  // (midpoints of longer intervals, each taking the next input dimension).
+  const void* bridge_ops;         // [n_steps - 1][4]: left weight, right weight, stddev, - (double, or float in FP32)
+  const uint8_t* bridge_counts;   // [n_steps]
   double bridge_sqrt_t, bridge_inv_sqrt_dt;
   uint32_t bridge;                // 1: normals come through the bridge
   uint32_t n_scen;                // scenario kernel: legs (0 elsewhere)
   // samplers
-  const uint32_t* halton_primes;
-  const double* halton_shifts;
+  const HaltonDim* halton;
+  const double* halton_weights;
   const LhsDim* lhs;
   // tiling and outputs
   uint32_t tile_units;     // units per tile

@@ -11,6 +11,7 @@ order 10 to 1000: 1e-11 relative leaves a factor of a hundred.
 import numpy as np
 import pytest
 
+from montepath_b200 import abi
 from montepath_b200.requests import make_request
 from oracle import oracle as O
 
@@ -75,3 +76,29 @@ def test_sobol_merton_extreme_intensities(backend, intensity, precision):
     got = backend.price_paths(r)
     rtol = 1e-11 if precision == "fp64_plain" else 1e-3
     assert np.allclose(got, ref, rtol=rtol, atol=rtol), float(np.max(np.abs(got - ref)))
+
+
+@pytest.mark.parametrize("sampling", ["randomized_halton", "latin_hypercube"])
+@pytest.mark.parametrize("n_paths,n_steps", [(1, 1), (2, 3), (8, 5), (9, 2), (243, 40), (65_536, 3), (65_537, 9)])
+def test_lattice_samples_at_digit_edges(backend, sampling, n_paths, n_steps):
+    """Point counts at powers of the small primes: the digit count of a
+    dimension changes there, and the strata are few.  FP64 normals to the bound
+    of the other sampler tests; FP32 ones within normcdfinvf's 5 ulp plus the
+    uniform's rounding (the slope of the inverse at 2^-24 is under 2^22)."""
+
+    code = abi.SAMPLINGS[sampling]
+    ref = O.generate_normals(code, 7, n_paths, n_steps)
+    got = backend.generate_normals(code, 7, n_paths, n_steps)
+    assert np.max(np.abs(got - ref) / np.maximum(1.0, np.abs(ref))) < 1e-13
+    f32 = backend.generate_normals(code, 7, n_paths, n_steps, fp32=True)
+    slope = 1.0 / np.maximum(np.exp(-0.5 * ref * ref) / np.sqrt(2.0 * np.pi), 1e-7)
+    assert np.all(np.abs(f32 - ref) < 2e-6 * np.maximum(1.0, np.abs(ref)) + 6e-8 * slope)
+
+
+def test_halton_wide_digit_products(backend):
+    """base^digits past 2^32 (2,700,000 points, primes above 1,626): FP32 against FP64 prices."""
+
+    kw = dict(method="stepwise", n_paths=2_700_000, n_steps=260, seed=3, sampling="randomized_halton")
+    a = backend.price(make_request("european_call", dict(kw, precision="fp32_path")))
+    b = backend.price(make_request("european_call", dict(kw, precision="fp64_plain")))
+    assert abs(a.price - b.price) < 0.01 * b.stderr, (a.price, b.price, b.stderr)
