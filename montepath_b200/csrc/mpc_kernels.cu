@@ -108,7 +108,7 @@ __device__ __forceinline__ uint64_t gf2_apply_shared(const uint64_t* table, uint
 // 2 * (idx / 2) draws, idx the unit's first normal in its chunk.
 template <int FAM>
 __device__ __forceinline__ void fused_unit_stream(const DevReq& q, uint64_t aligned, uint64_t idx, double& p, double& c) {
-  XorshiftFast src;
+  XorshiftPairs<float> src;
   src.start(aligned, idx);
   run_family<float, FAM>(q, src, p, c);
 }
@@ -486,8 +486,13 @@ int serve_loop_blocks_per_sm() {
 
 template <int FAM, int SMP>
 static int occ_t(int block) {
-  int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fused_kernel<FAM, SMP>, block, fused_dynamic_smem<SMP>());
+  static std::atomic<int> known[3];  // 128, 256, 512 threads; as lsm_capacity_t's
+  const int at = block == 128 ? 0 : block == 256 ? 1 : 2;
+  int n = known[at].load(std::memory_order_relaxed);
+  if (n <= 0) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fused_kernel<FAM, SMP>, block, fused_dynamic_smem<SMP>());
+    known[at].store(n, std::memory_order_relaxed);
+  }
   return n;
 }
 template <int SMP>
@@ -610,7 +615,7 @@ __device__ __forceinline__ void scen_gbm_step(const DevReq& q, Src& src, const f
   uint32_t st = 0;
   if constexpr (kPairSource<Src>) {
     for (; st + 2 <= n; st += 2) {
-      const float2 z = src.n32x2(st);
+      const auto z = src.n2(st);
       advance(z.x);
       advance(z.y);
     }
@@ -691,7 +696,7 @@ __device__ __forceinline__ void scen_heston(const DevReq& q, Src& src, const flo
   for (uint32_t st = 0; st < n; ++st) {
     float zv, zi;
     if constexpr (kPairSource<Src>) {
-      const float2 z = src.n32x2(2 * st);
+      const auto z = src.n2(2 * st);
       zv = z.x;
       zi = z.y;
     } else {
@@ -1145,6 +1150,15 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
+// x / 6 as x C + x c, C = 1/6 rounded and c the rest of 1/6: one multiplication
+// and one FMA (division by a constant known in advance, Brisebarre, Muller and
+// Raina 2004).  In FP32 this is the correctly rounded quotient (checked for
+// every mantissa); in FP64 it is within an ulp of it.
+__device__ __forceinline__ float sixth(float x) { return fmaf(x, 0.16666667f, x * -4.967053731882189e-09f); }
+__device__ __forceinline__ double sixth(double x) {
+  return fma(x, 0.16666666666666666, x * 9.25185853854297e-18);
+}
+
 template <class Real>
 __device__ __forceinline__ void laguerre4(Real x, Real b[4]) {
   // laguerre_lsm_basis (cpu.rs:7667-7682); degrees above `degree` are unused
@@ -1152,14 +1166,24 @@ __device__ __forceinline__ void laguerre4(Real x, Real b[4]) {
   b[0] = (Real)1;
   b[1] = (Real)1 - x;
   b[2] = (Real)1 - (Real)2 * x + (Real)0.5 * x2;
-  b[3] = (Real)1 - (Real)3 * x + (Real)1.5 * x2 - x3 / (Real)6;
+  b[3] = (Real)1 - (Real)3 * x + (Real)1.5 * x2 - sixth(x3);
+}
+
+// 1 / x to an ulp or two by Newton's iteration from the hardware's 20-bit
+// approximation (|x| is above the solve's 1e-12 pivot threshold).
+__device__ __forceinline__ double newton_reciprocal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
 }
 
 // solve_lsm_normal_equations (cpu.rs:7684-7736) for a compile-time size:
 // Gauss-Jordan with partial pivoting in FP64, the reference's operations in
-// its order, with every index static (the pivot row swap is a predicated exchange), so the
-// system stays in registers.
-template <int DIM, bool RECIP = false>
+// its order but with each pivot row scaled by the pivot's reciprocal, every
+// index static (the pivot row swap is a predicated exchange), so the system
+// stays in registers.
+template <int DIM>
 __device__ __forceinline__ bool solve_fixed(double a[4][4], double rhs[4]) {
 #pragma unroll
   for (int piv = 0; piv < DIM; ++piv) {
@@ -1178,7 +1202,7 @@ __device__ __forceinline__ bool solve_fixed(double a[4][4], double rhs[4]) {
     for (int row = piv + 1; row < DIM; ++row) {
       if (row == best) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = piv; c < DIM; ++c) {
           const double t = a[piv][c];
           a[piv][c] = a[row][c];
           a[row][c] = t;
@@ -1188,30 +1212,21 @@ __device__ __forceinline__ bool solve_fixed(double a[4][4], double rhs[4]) {
         rhs[row] = t;
       }
     }
-    const double pv = a[piv][piv];
-    if constexpr (RECIP) {
-      const double ip = 1.0 / pv;
+    const double ip = newton_reciprocal(a[piv][piv]);
 #pragma unroll
-      for (int c = piv; c < DIM; ++c) a[piv][c] *= ip;
-      rhs[piv] *= ip;
-    } else {
-#pragma unroll
-      for (int c = piv; c < DIM; ++c) a[piv][c] /= pv;
-      rhs[piv] /= pv;
-    }
+    for (int c = piv + 1; c < DIM; ++c) a[piv][c] *= ip;
+    rhs[piv] *= ip;
 #pragma unroll
     for (int row = 0; row < DIM; ++row) {
       if (row == piv) continue;
       const double f = a[row][piv];
-      if (f == 0.0) continue;
 #pragma unroll
-      for (int c = piv; c < DIM; ++c) a[row][c] -= f * a[piv][c];
+      for (int c = piv + 1; c < DIM; ++c) a[row][c] -= f * a[piv][c];
       rhs[row] -= f * rhs[piv];
     }
   }
   return true;
 }
-
 
 constexpr int kLsmBlock = (int)kLsmThreads;
 
@@ -1220,7 +1235,10 @@ constexpr int kLsmMom = 15;  // 10 unique A^T A, 4 A^T b, ITM count
 
 // Records the first failed self-check of an LSM job (code and index).
 __device__ __noinline__ void lsm_report(const LsmArgs& a, int code, uint64_t index) {
-  if (atomicCAS(a.error, 0, code) == 0) *a.diag = (unsigned long long)index;
+  if (atomicCAS(a.error, 0, code) == 0) {
+    *(volatile unsigned long long*)a.diag = (unsigned long long)index;  // status and diag: mapped host memory
+    *(volatile int*)a.status = code;
+  }
 }
 __device__ __forceinline__ bool lsm_ok(const LsmArgs& a, uint64_t index, uint64_t len, int code) {
   if (index < len) return true;
@@ -1262,9 +1280,9 @@ __device__ __forceinline__ uint32_t reduce_scatter16_index(uint32_t lane) {
 // of the round at once and re-reads (bounded) only those still empty, with no
 // fence, counter or separate poll between the write and the read.  Then every
 // block sums the partials itself in the same fixed order (thread t: moment
-// t % 16 over blocks t / 16, t / 16 + 32, ...; the lane groups' sums by
-// shuffles, then a fixed shuffle tree per moment over the 16 warps) and solves
-// the normal equations in thread 0: the same operations on the same data, so
+// t % 16 over blocks t / 16, t / 16 + 32, ...; the lane groups' sums by a
+// shuffle, then lane m of warp 0 over the 16 warps) and solves the normal
+// equations in thread 0: the same operations on the same data, so
 // every block holds the same coefficients, with no publication round trip
 // after the solve.  The FP32 path scales each pivot row by the pivot's
 // reciprocal instead of dividing every entry (the FP64 path divides, as the
@@ -1284,12 +1302,19 @@ __device__ __forceinline__ void st_relaxed_f64(double* p, double x) {
   if (v == kLsmEmpty) v = 0x7FF8000000000001ull;  // a NaN with the marker's bits: keep it a NaN
   asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-template <bool RECIP>
-__device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, uint32_t lb, uint32_t round,
-                                                 int coeffs, double* fold, double* s_mom, double* s_beta, int* s_ok) {
-  __shared__ int s_bad;
-  if (threadIdx.x == 0) s_bad = 0;
-  __syncthreads();
+// Sums of the 16 warps' values of moment `mom` (0..15), in two fixed chains.
+__device__ __forceinline__ double sum_warps16(const double* rows, uint32_t mom) {
+  double e = rows[mom], o = rows[17 + mom];
+#pragma unroll
+  for (int w = 2; w < 16; w += 2) {
+    e += rows[w * 17 + mom];
+    o += rows[(w + 1) * 17 + mom];
+  }
+  return e + o;
+}
+// s_bad: shared flag, 0 until a wait fails (then the job's blocks all leave).
+__device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, uint32_t round, int coeffs,
+                                                 double* fold, double* s_mom, double* s_beta, int* s_ok, int* s_bad) {
   const uint64_t base_at = (uint64_t)round * nb * 16;
   const uint32_t mom = threadIdx.x & 15u, lane_grp = threadIdx.x >> 4, n_grp = blockDim.x >> 4;
   double acc = 0.0;
@@ -1316,12 +1341,12 @@ __device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, 
         }
         if (!pending) break;
         if (*((volatile int*)a.error) != 0) {
-          s_bad = 1;
+          *s_bad = 1;
           break;
         }
         if (global_ns() - start > a.timeout_ns) {
-          atomicCAS(a.error, 0, kLsmErrTimeout);
-          s_bad = 1;
+          lsm_report(a, kLsmErrTimeout, round);
+          *s_bad = 1;
           break;
         }
       }
@@ -1329,21 +1354,15 @@ __device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, 
       for (int i = 0; i < kBatch; ++i) acc += __longlong_as_double((long long)v[i]);
     }
   }
-  __syncthreads();
-  if (s_bad) return false;
+  __syncwarp();
   acc += __shfl_xor_sync(0xffffffffu, acc, 16);  // the warp's two lane groups
   if ((threadIdx.x & 31u) < 16u) fold[(threadIdx.x >> 5) * 17 + mom] = acc;
   __syncthreads();
-  if (threadIdx.x < 256u) {  // 16 warps (512-thread blocks): moment t / 16 over warp t % 16
-    const uint32_t mo = threadIdx.x >> 4, w = threadIdx.x & 15u;
-    double t = mo < (uint32_t)kLsmMom ? fold[w * 17 + mo] : 0.0;
-    t += __shfl_xor_sync(0xffffffffu, t, 8);
-    t += __shfl_xor_sync(0xffffffffu, t, 4);
-    t += __shfl_xor_sync(0xffffffffu, t, 2);
-    t += __shfl_xor_sync(0xffffffffu, t, 1);
-    if (w == 0 && mo < (uint32_t)kLsmMom) s_mom[mo] = t;
+  if (*s_bad) return false;
+  if (threadIdx.x < 32u) {
+    if (threadIdx.x < (uint32_t)kLsmMom) s_mom[threadIdx.x] = sum_warps16(fold, threadIdx.x);
+    __syncwarp();
   }
-  __syncthreads();
   if (threadIdx.x == 0) {
     double ata[4][4], atb[4];
     int idx = 0;
@@ -1357,16 +1376,9 @@ __device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, 
       }
 #pragma unroll
     for (int r = 0; r < 4; ++r) atb[r] = s_mom[10 + r];
-    // the reference zeroes rows/columns beyond the basis degree
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (r < coeffs) continue;
-      atb[r] = 0.0;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) ata[r][c] = ata[c][r] = 0.0;
-    }
+    // rows and columns past the basis degree are never read
     int ok = s_mom[14] >= (double)coeffs ? 1 : 0;
-    if (ok) ok = (coeffs == 2 ? solve_fixed<2, RECIP>(ata, atb) : coeffs == 3 ? solve_fixed<3, RECIP>(ata, atb) : solve_fixed<4, RECIP>(ata, atb)) ? 1 : 0;
+    if (ok) ok = (coeffs == 2 ? solve_fixed<2>(ata, atb) : coeffs == 3 ? solve_fixed<3>(ata, atb) : solve_fixed<4>(ata, atb)) ? 1 : 0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) s_beta[r] = (ok && r < coeffs) ? atb[r] : 0.0;
     *s_ok = ok;
@@ -1378,6 +1390,13 @@ __device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, 
 // One 512-thread block per SM: the same warps per SM as two 256-thread
 // blocks, but half the block partials to fold per date (the per-date
 // cross-block round is this kernel's critical path).
+// Bound by the latency of the date rounds (moments, one exchange through L2,
+// the solve, the exercise pass, at 16 warps an SM) and by the path generation
+// before them.  524,288 paths x 50 dates on a B200, before -> now: generation 96
+// -> 76 us (pairs of normals), a round 4.84 -> 4.22 us in FP32 and 7.86 -> 5.86
+// in FP64 (x^3 / 6 without a division, Newton reciprocals in the solve, three
+// block barriers a round instead of five, and the generation loop not unrolled:
+// with eight copies of the sampling code a round took 5.8 us).
 template <class Real, int SMP>
 __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(const LsmArgs* __restrict__ jobs, uint32_t n_jobs, SrcCtx ctx) {
   __shared__ double red[kLsmBlock / 32][5];
@@ -1386,12 +1405,14 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(const LsmArgs* __rest
   __shared__ int s_ok;
   __shared__ uint32_t s_job;
   __shared__ double s_red15[kLsmBlock / 32][17];
-  __shared__ double s_fold[kLsmBlock];  // 16 lanes x 16 moments of the last block's fold
+  __shared__ double s_fold[kLsmBlock / 32 * 17];  // [warp][moment] of the fold over the blocks
+  __shared__ int s_bad;
   __shared__ Real s_disc[512];
   if (threadIdx.x == 0) {
     uint32_t j = 0;
     while (j + 1 < n_jobs && blockIdx.x >= jobs[j + 1].block_first) ++j;
     s_job = j;
+    s_bad = 0;
   }
   __syncthreads();
   const LsmArgs a = jobs[s_job];
@@ -1428,29 +1449,48 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(const LsmArgs* __rest
   // T^(nthreads x steps) draws (nthreads is even, so the pair alignment of
   // the start carries over), 16 table lookups instead of a full seek.
   uint64_t aligned = 0;
-#pragma unroll
+#pragma unroll 1  // one copy of the sampling code: unrolled, it pushes the date loop out of the instruction cache
   for (int j = 0; j < kLsmMaxP; ++j) {
     const uint64_t path = gtid + (uint64_t)j * nthreads;
-    cash[j] = 0;
-    exd[j] = steps;
     if (path >= n) continue;
-    Source<SMP> src;
+    // the path's last element bounds all of them
+    if (!lsm_ok(a, (uint64_t)(steps - 1) * n + path, a.paths_len, kLsmErrPaths)) continue;
+    Real* out = paths + path;
+    Real s = (Real)a.s0;
+    auto advance = [&](const Real z) {
+      s *= ex<Real>(drift + vol * z);  // multiplicative update as cpu.rs:3829-3830
+      *out = s;
+      out += n;
+    };
     if constexpr (SMP == SMP_XORSHIFT) {
       const uint64_t idx = path * steps;
       aligned = (j == 0 || a.stride_jump == nullptr)
                     ? xorshift_jump(ctx.jump, XorshiftStream::first_state(a.seed), 2 * (idx >> 1))
                     : gf2_apply(a.stride_jump, aligned);
-      src.st.seek_aligned(aligned, idx, sizeof(Real) == 4);
+      XorshiftPairs<Real> src;
+      src.start(aligned, idx);
+      uint32_t st = 0;
+      for (; st + 2 <= steps; st += 2) {
+        const auto z = src.n2(st);
+        advance(z.x);
+        advance(z.y);
+      }
+      if (st < steps) advance(src.next());
     } else {
+      Source<SMP> src;
       src.template begin<sizeof(Real) == 8>(q, ctx, path);
+      for (uint32_t st = 0; st < steps; ++st) advance(normal<Real>(src, st));
     }
-    Real s = (Real)a.s0;
-    for (uint32_t st = 1; st <= steps; ++st) {
-      const Real z = normal<Real>(src, st - 1);
-      s *= ex<Real>(drift + vol * z);  // multiplicative update as cpu.rs:3829-3830
-      const uint64_t idx = (uint64_t)(st - 1) * n + path;
-      if (lsm_ok(a, idx, a.paths_len, kLsmErrPaths)) paths[idx] = s;
-    }
+  }
+#pragma unroll
+  for (int j = 0; j < kLsmMaxP; ++j) {  // maturity cashflows, from the thread's own stores
+    const uint64_t path = gtid + (uint64_t)j * nthreads;
+    cash[j] = (Real)0;
+    exd[j] = steps;
+    if (path >= n) continue;
+    const uint64_t at = (uint64_t)(steps - 1) * n + path;
+    if (!lsm_ok(a, at, a.paths_len, kLsmErrPaths)) continue;
+    const Real s = paths[at];
     cash[j] = k - s > (Real)0 ? k - s : (Real)0;
   }
   uint32_t regressions = 0, round = 0;
@@ -1474,15 +1514,12 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(const LsmArgs* __rest
     if (step == 0 || step > steps) {
       if (threadIdx.x == 0) lsm_report(a, kLsmErrSched, step);
     }
-    double m[kLsmMom];
+    // Each thread sums the 15 moments of its own <= kLsmMaxP paths, the FP32
+    // path in FP32 (the warps too; FP64 takes over from the warp sums): 10 of
+    // A^T A (the first is the count, as the basis starts with 1), 4 of A^T b.
+    Real m[14];
 #pragma unroll
-    for (int i = 0; i < kLsmMom; ++i) m[i] = 0.0;
-    // FP32 path: each thread sums its own <= kLsmMaxP paths in FP32 and the
-    // warp sums them in FP32; FP64 takes over from the warp sums (block,
-    // cross-block)
-    float mf[kLsmMom];
-#pragma unroll
-    for (int i = 0; i < kLsmMom; ++i) mf[i] = 0.0f;
+    for (int i = 0; i < 14; ++i) m[i] = (Real)0;
     Real sv[kLsmMaxP];
 #pragma unroll
     for (int j = 0; j < kLsmMaxP; ++j) sv[j] = sv_next[j];
@@ -1491,75 +1528,43 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(const LsmArgs* __rest
       const uint64_t path = gtid + (uint64_t)j * nthreads;
       if (path >= n || step == 0 || step > steps) continue;
       const Real s = sv[j];
-      const Real imm = k - s;
-      if (!(imm > (Real)0)) continue;
+      if (!(k - s > (Real)0)) continue;
       if (exd[j] < step || exd[j] > steps) {
         lsm_report(a, kLsmErrDisc, exd[j]);
         continue;
       }
-      const Real cont = cash[j] * s_disc[exd[j] - step];
+      const Real c = cash[j] * s_disc[exd[j] - step];
       Real b[4];
       laguerre4<Real>(s * inv_k, b);
       int idx = 0;
-      if constexpr (sizeof(Real) == 4) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-          for (int c = r; c < 4; ++c) {
-            mf[idx] = fmaf(b[r], b[c], mf[idx]);
-            ++idx;
-          }
+        for (int t = r; t < 4; ++t) {
+          m[idx] = fma(b[r], b[t], m[idx]);
+          ++idx;
+        }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) mf[10 + r] = fmaf(b[r], cont, mf[10 + r]);
-        mf[14] += 1.0f;
-      } else {
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = r; c < 4; ++c) m[idx++] += (double)(b[r] * b[c]);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) m[10 + r] += (double)(b[r] * cont);
-        m[14] += 1.0;
-      }
+      for (int r = 0; r < 4; ++r) m[10 + r] = fma(b[r], c, m[10 + r]);
     }
-    // block reduction of the 15 moments: warp sums by reduce-scatter (the
-    // FP32 path reduces the thread sums in FP32 across the warp, and FP64
-    // takes over from the warp sums), then a fixed tree folds the warps
+    // block reduction: warp sums by reduce-scatter, then lane m of warp 0 over
+    // the 16 warps; the slot's own value marks its arrival (lsm_gather_solve)
     const uint64_t part_at = ((uint64_t)round * nb + lb) * 16;
     {
-      double w;
-      if constexpr (sizeof(Real) == 4) {
-        float mv[16];
+      Real mv[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) mv[i] = i < kLsmMom ? mf[i] : 0.0f;
-        w = (double)warp_reduce_scatter16(mv);
-      } else {
-        double mv[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) mv[i] = i < kLsmMom ? m[i] : 0.0;
-        w = warp_reduce_scatter16(mv);
-      }
+      for (int i = 0; i < 16; ++i) mv[i] = i < 14 ? m[i] : i == 14 ? m[0] : (Real)0;
+      const double w = (double)warp_reduce_scatter16(mv);
       const uint32_t lane = threadIdx.x & 31u;
       if ((lane & 1u) == 0) s_red15[threadIdx.x >> 5][reduce_scatter16_index(lane)] = w;
     }
     __syncthreads();
-    if (threadIdx.x < 256u) {
-      // moment m = t / 16 over the 16 warps w = t % 16: a shuffle tree per
-      // 16-lane group
-      const uint32_t mo = threadIdx.x >> 4, w = threadIdx.x & 15u;
-      double t = mo < (uint32_t)kLsmMom ? s_red15[w][mo] : 0.0;
-      t += __shfl_xor_sync(0xffffffffu, t, 8);
-      t += __shfl_xor_sync(0xffffffffu, t, 4);
-      t += __shfl_xor_sync(0xffffffffu, t, 2);
-      t += __shfl_xor_sync(0xffffffffu, t, 1);
-      // the slot's own value marks its arrival (lsm_gather_solve)
-      if (w == 0 && mo < (uint32_t)kLsmMom && lsm_ok(a, part_at + mo, a.partials_len, kLsmErrPartials))
-        st_relaxed_f64(a.partials + part_at + mo, t);
-    }
+    if (threadIdx.x < (uint32_t)kLsmMom && lsm_ok(a, part_at + threadIdx.x, a.partials_len, kLsmErrPartials))
+      st_relaxed_f64(a.partials + part_at + threadIdx.x, sum_warps16(&s_red15[0][0], threadIdx.x));
     if (si > 0) load_date(si - 1);  // next date's values, in flight during the wait
     // Every block waits (bounded) for all blocks' partials of this date, then
     // sums them in block order and solves the normal equations itself.
-    if (!lsm_gather_solve<sizeof(Real) == 4>(a, nb, lb, round++, coeffs, s_fold, s_mom, s_beta, &s_ok)) return;
+    if (!lsm_gather_solve(a, nb, round++, coeffs, s_fold, s_mom, s_beta, &s_ok, &s_bad)) return;
     if (s_ok) {
       ++regressions;
       const Real b0 = (Real)s_beta[0], b1 = (Real)s_beta[1], b2 = (Real)s_beta[2], b3 = (Real)s_beta[3];
@@ -1629,10 +1634,16 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(const LsmArgs* __rest
 
 template <class Real, int SMP>
 static uint32_t lsm_capacity_t() {
-  int dev = 0, sms = 148, per_sm = 0;
+  // blocks per SM follow from the kernel's registers and shared memory (one
+  // architecture), so the first answer above zero stands
+  static std::atomic<int> known{0};
+  int dev = 0, sms = 148, per_sm = known.load(std::memory_order_relaxed);
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lsm_kernel<Real, SMP>, kLsmBlock, 0);
+  if (per_sm <= 0) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lsm_kernel<Real, SMP>, kLsmBlock, 0);
+    known.store(per_sm, std::memory_order_relaxed);
+  }
   return per_sm > 0 ? (uint32_t)(sms * per_sm) : 0u;
 }
 

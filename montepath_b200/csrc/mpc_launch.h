@@ -99,11 +99,11 @@ struct LsmArgs {
   void* paths;               // [n_steps][n_paths] float or double
   double* partials;          // [rounds][grid][16], every slot empty (all bits set) at launch
   double* final_partials;    // [grid][4]
-  double* out;               // [8]: n, sum, sumsq, early, maturity, regressions, -, -
-  unsigned* barrier;         // counter area (kLsmCounterBytes)
-  unsigned* done;            // last-block counter
-  int* error;                // first failure: kLsmErr* code (0 = none)
-  unsigned long long* diag;  // offending index of a failed self-check
+  double* out;               // [8] in mapped host memory: n, sum, sumsq, early, maturity, regressions, -, -
+  unsigned* done;            // last-block counter (zero before and after)
+  int* error;                // first failure: kLsmErr* code (0 = none), device memory
+  int* status;               // the same code, mapped host memory
+  unsigned long long* diag;  // offending index of a failed self-check, mapped host memory
   uint64_t timeout_ns;
   uint32_t block_first;      // this job's blocks in the batched launch
   uint32_t n_blocks;
@@ -134,9 +134,6 @@ cudaError_t launch_lsm_batch(const LsmArgs* d_jobs, uint32_t n_jobs, uint32_t to
 uint32_t lsm_capacity(int fp64, int sampler);
 constexpr uint32_t kLsmPathsPerThreadMax = 8;
 constexpr uint32_t kLsmThreads = 512;
-// Counter area of an LSM job (zeroed per launch): the last-block counter at
-// uint 4, the error code at uint 8 and its index at uint 10.
-constexpr size_t kLsmCounterBytes = 256;
 
 // Bump-and-revalue legs sharing every normal: one request q (GBM step,
 // GBM terminal or Heston; xorshift, Sobol or counter-hash samples; any

@@ -225,13 +225,6 @@ struct Source<SMP_XORSHIFT> {
     chunk_of(q, u, &seed, &local);
     st.seek(c.jump, seed, local * q.normals_per_unit, !FP64);
   }
-  // begin for the FP64 path with all 32 lanes of the warp together.
-  __device__ __forceinline__ void begin_warp(const DevReq& q, const SrcCtx& c, uint64_t u) {
-    uint64_t seed, local;
-    chunk_of(q, u, &seed, &local);
-    const uint64_t idx = local * q.normals_per_unit;
-    st.seek_aligned(xorshift_seek_warp(c.jump, seed, 2 * (idx >> 1)), idx, false);
-  }
   __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
   // Sequential stream: dimensions must be requested in increasing order.
   __device__ __forceinline__ float n32(uint32_t) { return st.normal_f32(); }
@@ -417,7 +410,7 @@ struct CounterFastT {
   }
   __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
   __device__ __forceinline__ float n32(uint32_t d) { return counter_normal_fast<HWCOS>(seed, unit, d); }
-  __device__ __forceinline__ float2 n32x2(uint32_t d) {
+  __device__ __forceinline__ float2 n2(uint32_t d) {
     return counter_normal_pair<HWCOS>(base ^ (d * 2891336453u), base ^ ((d + 1u) * 2891336453u));
   }
   __device__ __forceinline__ float u32(uint32_t d) {
@@ -429,29 +422,39 @@ struct CounterFastT {
   }
 };
 
-// The MonteCarloRng stream for the fused kernels, a Box-Muller pair at a time:
-// no cached-normal branch per sample, and the sine branch a unit with an odd
-// start carries over stays in FP32.  Dimensions in increasing order.
-struct XorshiftFast {
+// The MonteCarloRng stream a Box-Muller pair at a time: no cached-normal branch
+// per sample, and the sine branch a unit with an odd start carries over stays
+// in the path's precision.  Dimensions in increasing order.
+__device__ __forceinline__ float2 make_pair2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 make_pair2(double a, double b) { return make_double2(a, b); }
+template <class Real>
+struct XorshiftPairs {
   XorshiftStream st;
-  float carry;
+  Real carry;
   bool odd;  // the next normal is `carry`
-  __device__ __forceinline__ float2 pair() {
-    const float u1 = st.next_open01_f32(), u2 = st.next_open01_f32();
-    const float r = sqrt_ftz(neg2_log_fast(u1));
-    float s, c;
-    // hardware sine and cosine of 2 pi (u2 - 1/2) in [-pi, pi], where their
-    // documented error is 2^-21.4 absolute
-    __sincosf(6.28318548f * (u2 - 0.5f), &s, &c);
-    return make_float2(r * -c, r * -s);
+  __device__ __forceinline__ auto pair() {
+    if constexpr (sizeof(Real) == 4) {
+      const float u1 = st.next_open01_f32(), u2 = st.next_open01_f32();
+      const float r = sqrt_ftz(neg2_log_fast(u1));
+      float s, c;
+      // hardware sine and cosine of 2 pi (u2 - 1/2) in [-pi, pi], where their
+      // documented error is 2^-21.4 absolute
+      __sincosf(6.28318548f * (u2 - 0.5f), &s, &c);
+      return make_float2(r * -c, r * -s);
+    } else {
+      st.has_cached = false;
+      const double z = st.normal_f64();
+      return make_double2(z, st.cached);
+    }
   }
   // Starts from `aligned`, the state after 2 * (idx / 2) draws.
   __device__ __forceinline__ void start(uint64_t aligned, uint64_t idx) {
     st.state = aligned;
     odd = (idx & 1) != 0;
-    carry = 0.0f;
+    carry = (Real)0;
     if (odd) carry = pair().y;
   }
+  // All 32 lanes of the warp together.
   template <bool FP64>
   __device__ __forceinline__ void begin(const DevReq& q, const SrcCtx& c, uint64_t u) {
     uint64_t seed, local;
@@ -460,19 +463,21 @@ struct XorshiftFast {
     start(xorshift_seek_warp(c.jump, seed, 2 * (idx >> 1)), idx);
   }
   __device__ __forceinline__ void at_step(uint32_t, uint32_t) {}
-  __device__ __forceinline__ float n32(uint32_t) {
+  __device__ __forceinline__ Real next() {
     if (odd) {
       odd = false;
       return carry;
     }
-    const float2 z = pair();
+    const auto z = pair();
     odd = true;
     carry = z.y;
     return z.x;
   }
-  __device__ __forceinline__ float2 n32x2(uint32_t) {
-    const float2 z = pair();
-    const float2 out = odd ? make_float2(carry, z.x) : z;
+  __device__ __forceinline__ float n32(uint32_t) { return (float)next(); }
+  __device__ __forceinline__ double n64(uint32_t) { return (double)next(); }
+  __device__ __forceinline__ auto n2(uint32_t) {
+    const auto z = pair();
+    const auto out = odd ? make_pair2(carry, z.x) : z;
     carry = z.y;
     return out;
   }
@@ -486,13 +491,13 @@ constexpr bool kQuadSource<SobolQuad> = true;
 template <>
 constexpr bool kQuadSource<SobolPlain> = true;
 
-// Sources that give the normals of two consecutive dimensions at once (n32x2).
+// Sources that give the normals of two consecutive dimensions at once (n2).
 template <class S>
 constexpr bool kPairSource = false;
 template <bool HWCOS>
 constexpr bool kPairSource<CounterFastT<HWCOS>> = true;
-template <>
-constexpr bool kPairSource<XorshiftFast> = true;
+template <class Real>
+constexpr bool kPairSource<XorshiftPairs<Real>> = true;
 
 template <int FAM, int SMP>
 struct FusedUnitSource {
@@ -510,7 +515,7 @@ struct FusedUnitSource<FAM, SMP_COUNTER> {
 };
 template <int FAM>
 struct FusedUnitSource<FAM, SMP_XORSHIFT> {
-  using type = XorshiftFast;
+  using type = XorshiftPairs<float>;
 };
 
 template <class Real, class Src>
@@ -691,7 +696,7 @@ __device__ __forceinline__ void unit_gbm_step(const DevReq& q, Src& src, double&
     }
   } else if constexpr (kPairSource<Src>) {
     for (; s + 2 <= n; s += 2) {
-      const float2 z = src.n32x2(s);
+      const auto z = src.n2(s);
       advance(z.x);
       advance(z.y);
     }
@@ -803,7 +808,7 @@ __device__ __forceinline__ void unit_heston(const DevReq& q, Src& src, double& p
     }
   } else if constexpr (kPairSource<Src>) {
     for (; s < n; ++s) {
-      const float2 z = src.n32x2(2 * s);
+      const auto z = src.n2(2 * s);
       step(z.x, z.y);
     }
   }
@@ -925,7 +930,7 @@ __device__ __forceinline__ void sum_step_normals(Src& src, uint32_t n, Real zs[D
         for (int h = 0; h < 2; ++h) {  // two steps are D pairs whatever D's parity
 #pragma unroll
           for (int p = 0; p < D; ++p) {
-            const float2 z = src.n32x2(dim + 2 * p);
+            const auto z = src.n2(dim + 2 * p);
             part[(2 * p) % D] += z.x;
             part[(2 * p + 1) % D] += z.y;
           }
@@ -1036,7 +1041,7 @@ __device__ __forceinline__ void unit_mlmc(const DevReq& q, Src& src, double& pay
     uint32_t s = 0;
     if constexpr (kPairSource<Src>) {
       for (; s + 2 <= q.n_steps; s += 2) {
-        const float2 z = src.n32x2(s);
+        const auto z = src.n2(s);
         advance(z.x);
         advance(z.y);
       }
@@ -1067,7 +1072,7 @@ __device__ __forceinline__ void unit_mlmc(const DevReq& q, Src& src, double& pay
     uint32_t m = 0;
     if constexpr (kPairSource<Src>) {
       for (; m + 2 <= M; m += 2, j += 2) {
-        const float2 z = src.n32x2(j);
+        const auto z = src.n2(j);
         fine(z.x);
         fine(z.y);
       }

@@ -31,6 +31,10 @@ template <>
 struct PlainSource<SMP_SOBOL> {
   using type = SobolPlain;
 };
+template <>
+struct PlainSource<SMP_XORSHIFT> {
+  using type = XorshiftPairs<double>;
+};
 
 // Resident blocks the register allocation must allow: a basket keeps its
 // Cholesky factor and per-asset constants in registers.
@@ -71,10 +75,7 @@ __global__ void __launch_bounds__(kPlainBlock, plain_min_blocks(FAM)) plain_kern
     const bool valid = base + threadIdx.x < last;
     const uint64_t u = valid ? base + threadIdx.x : last - 1;
     typename PlainSource<SMP>::type src;
-    if constexpr (SMP == SMP_XORSHIFT)
-      src.begin_warp(q, ctx, u);
-    else
-      src.template begin<true>(q, ctx, u);
+    src.template begin<true>(q, ctx, u);
     double p, c;
     run_family<double, FAM>(q, src, p, c);
     if (!valid) continue;

@@ -1148,7 +1148,6 @@ int run_lsm_batch(mpc_context* ctx, const std::vector<const mpc_request_t*>& req
     std::vector<uint32_t> sched;
     std::vector<double> disc_pow;
     std::vector<uint64_t> stride_tab;  // pseudorandom sampler: nibble table of the per-thread path stride jump
-    std::vector<uint8_t> blob;         // host copy of the job's schedule, discount powers and stride table
     bool normalised;
     uint32_t degree, blocks;
     int fp64, sampler;
@@ -1221,90 +1220,88 @@ int run_lsm_batch(mpc_context* ctx, const std::vector<const mpc_request_t*>& req
       blocks += jobs[i].blocks;
       done[i] = true;
     }
-    // device arena layout per job: paths | sched | disc | partials (one slot row per date) | final | out | counters
+    // Device arena: the group's descriptors and tables (one copy in from pinned
+    // memory), the slot rows of every job (one fill), then per job the path
+    // matrix and the estimator partials.  Results and failures come back
+    // through mapped pinned memory; counters and error codes sit in a buffer of
+    // their own that is zero when allocated and after every launch that did
+    // not fail.
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    std::vector<size_t> offs;
-    size_t bytes = align(group.size() * sizeof(LsmArgs));
-    for (size_t i : group) {
-      const Job& j = jobs[i];
-      offs.push_back(bytes);
-      const size_t elem = j.fp64 ? 8 : 4;
-      bytes += align(j.args.n_paths * j.args.n_steps * elem) + align(j.sched.size() * 4) +
-               align(j.disc_pow.size() * 8) + align(256 * 8) + align(lsm_rounds(j.sched.size()) * j.blocks * 16 * 8) +
-               align(j.blocks * 4ull * 8) +
-               align(8 * 8) + align(kLsmCounterBytes);
-    }
-    void* arena = nullptr;
+    auto slot_bytes = [&](const Job& j) { return align(lsm_rounds(j.sched.size()) * j.blocks * 16 * 8); };
+    auto table_bytes = [&](const Job& j) { return align(j.sched.size() * 4) + align(j.disc_pow.size() * 8) + 256 * 8; };
+    const size_t args_bytes = align(group.size() * sizeof(LsmArgs));
+    size_t copy_bytes = args_bytes, slots_at = 0, bytes = 0;
+    for (size_t i : group) copy_bytes += table_bytes(jobs[i]);
+    slots_at = copy_bytes;
+    bytes = slots_at;
+    for (size_t i : group) bytes += slot_bytes(jobs[i]);
+    const size_t slots_end = bytes;
+    for (size_t i : group)
+      bytes += align(jobs[i].args.n_paths * jobs[i].args.n_steps * (jobs[i].fp64 ? 8 : 4)) + align(jobs[i].blocks * 4ull * 8);
+    // pinned: per job 8 doubles of results and 16 bytes {code, -, index}, then the copy in
+    const size_t back_bytes = align(group.size() * 80);
+    void *arena = nullptr, *counters = nullptr, *pin = nullptr;
     int st = scratch(ctx, "lsm_arena", bytes, &arena);
+    if (st == MPC_OK) st = scratch(ctx, "lsm_counters", group.size() * 16, &counters);
+    if (st == MPC_OK) st = pinned_staging(ctx, back_bytes + copy_bytes, &pin);
     if (st != MPC_OK) return st;
-    std::vector<uint8_t> host(align(group.size() * sizeof(LsmArgs)));
+    std::memset(pin, 0, back_bytes);
+    double* hout = static_cast<double*>(pin);
+    uint8_t* hdiag = reinterpret_cast<uint8_t*>(hout + group.size() * 8);
+    uint8_t* host = static_cast<uint8_t*>(pin) + back_bytes;
     uint8_t* base = static_cast<uint8_t*>(arena);
+    size_t table_at = args_bytes, slot_at = slots_at, rest_at = slots_end;
     uint32_t block_first = 0;
     for (size_t g = 0; g < group.size(); ++g) {
       Job& j = jobs[group[g]];
-      const size_t elem = j.fp64 ? 8 : 4;
-      size_t o = offs[g];
       LsmArgs& a = j.args;
-      a.paths = base + o;
-      o += align(a.n_paths * a.n_steps * elem);
-      {  // schedule | discount powers | stream stride table: one host-to-device copy
-        const size_t sched_b = align(j.sched.size() * 4), disc_b = align(j.disc_pow.size() * 8);
-        std::vector<uint8_t> blob(sched_b + disc_b + 256 * 8, 0);
-        std::memcpy(blob.data(), j.sched.data(), j.sched.size() * 4);
-        std::memcpy(blob.data() + sched_b, j.disc_pow.data(), j.disc_pow.size() * 8);
-        if (!j.stride_tab.empty()) std::memcpy(blob.data() + sched_b + disc_b, j.stride_tab.data(), 256 * 8);
-        a.sched = reinterpret_cast<const uint32_t*>(base + o);
-        a.disc_pow = reinterpret_cast<const double*>(base + o + sched_b);
-        a.stride_jump = j.stride_tab.empty() ? nullptr : reinterpret_cast<const uint64_t*>(base + o + sched_b + disc_b);
-        j.blob.swap(blob);  // kept alive until the stream synchronises below
-        MPC_CUDA(ctx, cudaMemcpyAsync(base + o, j.blob.data(), j.blob.size(), cudaMemcpyHostToDevice, ctx->stream));
-        h2d += j.blob.size();
-        o += sched_b + disc_b + align(256 * 8);
-      }
-      a.partials = reinterpret_cast<double*>(base + o);
-      // one slot row per exercise date, all marked empty (every byte 0xFF)
-      MPC_CUDA(ctx, cudaMemsetAsync(a.partials, 0xFF, lsm_rounds(j.sched.size()) * j.blocks * 16 * 8, ctx->stream));
-      o += align(lsm_rounds(j.sched.size()) * j.blocks * 16 * 8);
-      a.final_partials = reinterpret_cast<double*>(base + o);
-      o += align(j.blocks * 4ull * 8);
-      a.out = reinterpret_cast<double*>(base + o);
-      o += align(8 * 8);
-      // counters (zeroed per launch): block-done counter at 16, error code
-      // at 32, failed index at 40
-      a.barrier = reinterpret_cast<unsigned*>(base + o);
-      a.done = a.barrier + 4;
-      a.error = reinterpret_cast<int*>(a.barrier + 8);
-      a.diag = reinterpret_cast<unsigned long long*>(a.barrier + 10);
-      MPC_CUDA(ctx, cudaMemsetAsync(a.barrier, 0, kLsmCounterBytes, ctx->stream));
+      const size_t sched_b = align(j.sched.size() * 4), disc_b = align(j.disc_pow.size() * 8);
+      std::memcpy(host + table_at, j.sched.data(), j.sched.size() * 4);
+      std::memcpy(host + table_at + sched_b, j.disc_pow.data(), j.disc_pow.size() * 8);
+      if (!j.stride_tab.empty()) std::memcpy(host + table_at + sched_b + disc_b, j.stride_tab.data(), 256 * 8);
+      a.sched = reinterpret_cast<const uint32_t*>(base + table_at);
+      a.disc_pow = reinterpret_cast<const double*>(base + table_at + sched_b);
+      a.stride_jump = j.stride_tab.empty() ? nullptr : reinterpret_cast<const uint64_t*>(base + table_at + sched_b + disc_b);
+      table_at += table_bytes(j);
+      a.partials = reinterpret_cast<double*>(base + slot_at);
+      slot_at += slot_bytes(j);
+      a.paths = base + rest_at;
+      rest_at += align(a.n_paths * a.n_steps * (j.fp64 ? 8 : 4));
+      a.final_partials = reinterpret_cast<double*>(base + rest_at);
+      rest_at += align(j.blocks * 4ull * 8);
+      a.out = hout + g * 8;
+      a.status = reinterpret_cast<int*>(hdiag + g * 16);
+      a.diag = reinterpret_cast<unsigned long long*>(hdiag + g * 16 + 8);
+      a.done = static_cast<unsigned*>(counters) + 4 * g;
+      a.error = static_cast<int*>(counters) + 4 * g + 1;
       a.paths_len = a.n_paths * a.n_steps;
       a.partials_len = uint32_t(lsm_rounds(j.sched.size()) * j.blocks * 16u);
       a.final_len = j.blocks * 4u;
       a.block_first = block_first;
       a.n_blocks = j.blocks;
       block_first += j.blocks;
-      std::memcpy(host.data() + g * sizeof(LsmArgs), &a, sizeof(LsmArgs));
+      std::memcpy(host + g * sizeof(LsmArgs), &a, sizeof(LsmArgs));
     }
-    MPC_CUDA(ctx, cudaMemcpyAsync(base, host.data(), group.size() * sizeof(LsmArgs), cudaMemcpyHostToDevice,
-                                  ctx->stream));
-    h2d += group.size() * sizeof(LsmArgs);
+    MPC_CUDA(ctx, cudaMemcpyAsync(base, host, copy_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    // every slot marked empty (all bits set)
+    MPC_CUDA(ctx, cudaMemsetAsync(base + slots_at, 0xFF, slots_end - slots_at, ctx->stream));
+    h2d += copy_bytes;
+    d2h += group.size() * 80;
     MPC_CUDA(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
     cudaError_t e = launch_lsm_batch(reinterpret_cast<const LsmArgs*>(base), uint32_t(group.size()), block_first,
                                      fp64, sampler, ctx->tabs, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "LSM cooperative launch");
-    // pinned results: per job 8 doubles of output, then per job 16 bytes of
-    // {error code, pad, failed index} copied from the counters at byte 32
-    void* pin = nullptr;
-    if ((st = pinned_staging(ctx, group.size() * 80, &pin))) return st;
-    double* hout = static_cast<double*>(pin);
-    uint8_t* hdiag = reinterpret_cast<uint8_t*>(hout + group.size() * 8);
-    for (size_t g = 0; g < group.size(); ++g) {
-      const LsmArgs& a = jobs[group[g]].args;
-      MPC_CUDA(ctx, cudaMemcpyAsync(hout + g * 8, a.out, 8 * 8, cudaMemcpyDeviceToHost, ctx->stream));
-      MPC_CUDA(ctx, cudaMemcpyAsync(hdiag + g * 16, a.error, 16, cudaMemcpyDeviceToHost, ctx->stream));
-      d2h += 8 * 8 + 16;
-    }
     MPC_CUDA(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
     MPC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    for (size_t g = 0; g < group.size(); ++g) {
+      int code = 0;
+      std::memcpy(&code, hdiag + g * 16, sizeof(code));
+      if (code != 0) {  // a failed job leaves its counters as they were
+        MPC_CUDA(ctx, cudaMemsetAsync(counters, 0, group.size() * 16, ctx->stream));
+        MPC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        break;
+      }
+    }
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
     total_ms += ms;
