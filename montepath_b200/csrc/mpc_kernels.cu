@@ -1169,18 +1169,10 @@ __device__ __forceinline__ void laguerre4(Real x, Real b[4]) {
   b[3] = (Real)1 - (Real)3 * x + (Real)1.5 * x2 - sixth(x3);
 }
 
-// 1 / x to an ulp or two by Newton's iteration from the hardware's 20-bit
-// approximation (|x| is above the solve's 1e-12 pivot threshold).
-__device__ __forceinline__ double newton_reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-
 // solve_lsm_normal_equations (cpu.rs:7684-7736) for a compile-time size:
 // Gauss-Jordan with partial pivoting in FP64, the reference's operations in
-// its order but with each pivot row scaled by the pivot's reciprocal, every
+// its order but with each pivot row scaled by the pivot's reciprocal
+// (|pivot| > 1e-12), every
 // index static (the pivot row swap is a predicated exchange), so the system
 // stays in registers.
 template <int DIM>

@@ -11,7 +11,8 @@
 // pair of 131,072 paths x 256 steps on scrambled Sobol took 2,890 us
 // (generation 1,185 + 1,303, most of it the inverse normal's tail run by whole
 // warps for single lanes and the Merton dimensions drawn but not used) against
-// 605 us here.  Bound by FP64 issue.
+// 552 us here.  Bound by issue and FP64 latency together (issue slots 0.69, FP64
+// pipe 0.45 of peak in the Heston kernel at 27 warps an SM).
 #pragma once
 
 #include <cuda_runtime.h>

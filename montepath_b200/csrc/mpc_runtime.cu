@@ -1860,29 +1860,29 @@ enum CostRow : int {
   ROW_BRIDGE,
   ROW_COUNT
 };
-// The GBM stepwise Sobol cells are not the measured 4.3e11 and 2.2e11: the
+// The GBM stepwise Sobol cells are not the measured 4.8e11 and 2.7e11: the
 // planner's order is pinned to an estimate of at least five fused runtimes for
 // an FP64 one of that shape, so the two stand apart by that, each within the
 // factor of two the model answers for; mpc_calibrate_cost measures both.
 const RateRow kRates[ROW_COUNT] = {
-    {{3.72e11, 3.25e11, 6.00e11, 9.05e10}, {1.85e11, 1.83e11, 1.16e11, 6.05e10}},  // GBM stepwise (Sobol: see below)
-    {{3.48e11, 2.93e11, 4.15e11, 8.84e10}, {1.44e11, 1.42e11, 1.75e11, 5.51e10}},  // arithmetic Asian
-    {{5.4e10, 2.09e10, 1.73e10, 1.11e10}, {1.33e10, 3.94e10, 3.58e10, 1.29e10}},  // GBM terminal (pseudorandom FP32: + kTerminalFixedMs)
-    {{2.51e11, 1.96e11, 2.70e11, 5.37e10}, {9.46e10, 8.77e10, 1.06e11, 3.58e10}},  // Heston
-    {{1.05e11, 1.05e11, 2.88e11, 4.30e10}, {7.51e10, 7.51e10, 1.49e11, 4.70e10}},  // Merton stepwise
-    {{1.72e10, 1.79e10, 1.52e10, 7.09e9}, {1.72e10, 2.92e10, 2.73e10, 7.37e9}},    // Merton terminal
-    {{1.29e10, 1.53e10, 1.48e10, 7.87e9}, {1.10e10, 2.46e10, 2.02e10, 6.26e9}},    // 2-asset basket
-    {{1.49e11, 1.49e11, 1.49e11, 1.49e11}, {9.73e10, 9.73e10, 9.73e10, 9.73e10}},  // GBM stepwise, bridge
+    {{5.43e11, 4.92e11, 6.75e11, 2.45e11}, {1.89e11, 1.74e11, 1.32e11, 9.54e10}},  // GBM stepwise (Sobol: see above)
+    {{4.90e11, 4.42e11, 4.74e11, 2.37e11}, {1.53e11, 1.37e11, 1.97e11, 8.24e10}},  // arithmetic Asian
+    {{6.1e10, 2.88e10, 2.29e10, 2.36e10}, {1.28e10, 3.76e10, 3.49e10, 2.22e10}},   // GBM terminal (pseudorandom FP32: + kTerminalFixedMs)
+    {{3.16e11, 2.10e11, 2.83e11, 1.35e11}, {9.50e10, 8.50e10, 1.23e11, 5.51e10}},  // Heston
+    {{1.09e11, 1.09e11, 3.07e11, 8.50e10}, {7.52e10, 7.52e10, 1.65e11, 8.60e10}},  // Merton stepwise
+    {{1.70e10, 2.33e10, 2.05e10, 1.74e10}, {1.70e10, 2.73e10, 2.74e10, 1.33e10}},  // Merton terminal
+    {{2.45e10, 2.18e10, 1.96e10, 1.79e10}, {1.17e10, 2.75e10, 2.73e10, 1.38e10}},  // 2-asset basket
+    {{1.59e11, 1.59e11, 1.59e11, 1.59e11}, {1.16e11, 1.16e11, 1.16e11, 1.16e11}},  // GBM stepwise, bridge
 };
 // FP32 pseudorandom terminal GBM: each thread's first path of a tile takes a
 // full stream seek and its later paths one table jump each, so the time has
 // an intercept (about one full seek per resident thread, scaled down for
 // requests with fewer paths than resident threads) beside the per-path
-// rate (fit to 2,097,152 and 4,194,304 paths on a B200: 0.082 and 0.119 ms).
-const double kTerminalFixedMs = 0.046;
-const double kLsmFixedMs = 0.22, kLsmRate = 1.7e11; // 49 cross-block date rounds, then path-steps
-                                                      // (fit to 524,288 paths x 50 dates, FP32: 0.37 ms)
-const double kCallOverheadMs = 0.035;               // events, copies, one launch
+// rate (fit to 2,097,152 and 4,194,304 paths on a B200: 0.051 and 0.085 ms).
+const double kTerminalFixedMs = 0.017;
+const double kLsmFixedMs = 0.17, kLsmRate = 2.2e11; // 49 cross-block date rounds, then path-steps
+                                                      // (fit to 524,288 paths x 50 dates, FP32: 0.284 ms)
+const double kCallOverheadMs = 0.015;               // events, one launch
 const double kFirstCallMs = 2.0;                    // tables and buffers of a new shape
 const int kCostColumns = 4;
 const int kCalibrationSampling[kCostColumns] = {MPC_SAMPLING_PSEUDORANDOM, MPC_SAMPLING_COUNTER_HASH,
