@@ -1,7 +1,6 @@
 // mpc_device.cuh -- device-side generators, inverse CDF and reductions of the
 // B200 Monte Carlo backend.  Everything here is evaluated in registers inside
-// the fused pricing kernels; no sample is materialised unless the request is
-// an FP64-plain one.
+// the pricing kernels; no sample is written to memory.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -553,6 +552,32 @@ __device__ __forceinline__ double halton_f32(uint64_t index, const HaltonDim* __
   }
   const double shifted = fma(reversed, tail.x, tail.y);
   return shifted >= 1.0 ? shifted - 1.0 : shifted;
+}
+// Two consecutive dimensions: the same values, both digit chains in one loop
+// (bases rise with the dimension, so the second has no more digits).
+__device__ __forceinline__ double2 halton_f32_pair(uint64_t index, const HaltonDim* __restrict__ dim) {
+  const uint4 ha = __ldg(reinterpret_cast<const uint4*>(dim)), hb = __ldg(reinterpret_cast<const uint4*>(dim + 1));
+  if (((ha.z | hb.z) & 0xFF0000u) || !(ha.z & 0xFF00u) || !(hb.z & 0xFF00u))
+    return make_double2(halton_f32(index, dim), halton_f32(index, dim + 1));
+  const double2 ta = __ldg(reinterpret_cast<const double2*>(dim) + 1);
+  const double2 tb = __ldg(reinterpret_cast<const double2*>(dim + 1) + 1);
+  const uint32_t sa = ha.z & 0xFFu, sb = hb.z & 0xFFu, da = (ha.z >> 8) & 0xFFu, db = (hb.z >> 8) & 0xFFu;
+  uint32_t na = (uint32_t)index, nb = na, ra = 0, rb = 0, k = 0;
+  for (; k < db; ++k) {
+    const uint32_t qa = __umulhi(na, ha.y) >> sa, qb = __umulhi(nb, hb.y) >> sb;
+    ra = ra * ha.x + (na - qa * ha.x);
+    rb = rb * hb.x + (nb - qb * hb.x);
+    na = qa;
+    nb = qb;
+  }
+  for (; k < da; ++k) {
+    const uint32_t qa = __umulhi(na, ha.y) >> sa;
+    ra = ra * ha.x + (na - qa * ha.x);
+    na = qa;
+  }
+  const double a = fma(__hiloint2double(0x43300000, (int)ra) - 4503599627370496.0, ta.x, ta.y);
+  const double b = fma(__hiloint2double(0x43300000, (int)rb) - 4503599627370496.0, tb.x, tb.y);
+  return make_double2(a >= 1.0 ? a - 1.0 : a, b >= 1.0 ? b - 1.0 : b);
 }
 
 __device__ __forceinline__ double open01_from_u64(uint64_t v) {

@@ -33,6 +33,27 @@ def test_units_by_pairs(backend, workload, kw, sampling, n_paths, n_steps, threa
     check(backend, workload, dict(kw, sampling=sampling, n_paths=n_paths, n_steps=n_steps, n_threads=threads, seed=13))
 
 
+@pytest.mark.parametrize("workload", ["european_call", "arithmetic_asian_call", "lookback_call"])
+@pytest.mark.parametrize("sampling", ["randomized_halton", "latin_hypercube"])
+@pytest.mark.parametrize("n_paths,n_steps", [(1, 1), (8, 2), (243, 5), (8003, 36)])
+def test_lattice_units_by_pairs(backend, workload, sampling, n_paths, n_steps):
+    """Pairs of dimensions (of different digit counts, and a last single one)
+    against paths of the same FP32 normals, which the sampler gives one at a
+    time: only the path's own FP32 rounding is between them."""
+    req = make_request(workload, dict(method="stepwise", sampling=sampling, n_paths=n_paths, n_steps=n_steps, seed=13,
+                                      precision="fp32_path"))
+    z = backend.generate_normals(req.sampling, 13, n_paths, n_steps, fp32=True).astype(np.float64)
+    z = z.reshape(n_paths, n_steps)
+    dt = req.t / n_steps
+    log = np.log(req.s0) + np.cumsum((req.r - 0.5 * req.sigma**2) * dt + req.sigma * np.sqrt(dt) * z, axis=1)
+    spot = np.exp(log)
+    level = {"european_call": spot[:, -1], "arithmetic_asian_call": spot.mean(axis=1),
+             "lookback_call": np.maximum(spot.max(axis=1), req.s0)}[workload]
+    ref = np.exp(-req.r * req.t) * np.maximum(level - req.k, 0.0)
+    got = backend.price_paths(req)
+    assert np.allclose(got, ref, rtol=1e-3, atol=2e-3), float(np.max(np.abs(got - ref)))
+
+
 @pytest.mark.parametrize("assets", range(1, 9))
 @pytest.mark.parametrize("n_steps", [1, 2, 5])
 @pytest.mark.parametrize("sampling,technique", [("pseudorandom", "standard"), ("counter_hash", "antithetic")])
