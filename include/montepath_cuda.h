@@ -92,7 +92,7 @@ typedef enum mpc_sampling {
 } mpc_sampling_t;
 
 typedef enum mpc_precision {
-  MPC_PRECISION_FP64_PLAIN = 0, /* one request per launch, FP64, materialised normals */
+  MPC_PRECISION_FP64_PLAIN = 0, /* one request per launch, FP64 samples and paths */
   MPC_PRECISION_FP32_PATH = 1   /* fused FP32 path arithmetic, FP64 accumulation */
 } mpc_precision_t;
 
@@ -365,8 +365,10 @@ int mpc_prepare(mpc_context_t* ctx, const mpc_request_t* req, mpc_artifact_t* ou
 int mpc_price(mpc_context_t* ctx, const mpc_request_t* req, mpc_result_t* out);
 /* Prices n requests: the FP32-path requests in one persistent launch per
  * (sampler, family) group, the FP64-plain requests one launch sequence each,
- * LSM and MLMC requests in shared launches.  When a fused batch of the same
- * shape (sizes, launch shapes, buffers) comes twice in a row, the second call
+ * LSM and MLMC requests in shared launches.  Up to four requests of a group
+ * go in the launch's own parameters (no copy in, no memset, no copy out).  A
+ * batch with a larger group copies its descriptors; when one of the same shape
+ * (sizes, launch shapes, buffers) comes twice in a row, the second call
  * captures its copy/launch sequence in a CUDA graph and later calls of that
  * shape replay the graph (one launch call). */
 int mpc_price_batch(mpc_context_t* ctx, const mpc_request_t* reqs, size_t n, mpc_result_t* out);

@@ -298,7 +298,8 @@ bool merton_stream_request(const mpc_request_t& r) {
 }
 
 uint64_t estimate_bytes(const mpc_request_t& r) {
-  // Fused: tile partials only.  Plain: materialised samples + payoff buffers.
+  // Fused: tile partials only.  Plain: every sample and payoff counted at 8
+  // bytes, the documented admission size (the kernels keep less).
   if (r.workload == MPC_WORKLOAD_ASIAN_MLMC) {
     uint64_t total = 0, fine = r.base_steps;
     for (uint32_t l = 0; l < r.levels && l < MPC_MAX_LEVELS; ++l) {
@@ -324,8 +325,8 @@ uint64_t estimate_bytes(const mpc_request_t& r) {
     dims = 1;
   uint64_t partials = (units / 256 + 1) * 64 + 1024;
   if (merton_stream_request(r)) {
-    // stream outputs and jump bits (3 positions per path + spare segments),
-    // segment maps and states, path starts, payoffs
+    // the documented size: 8 bytes per stream position (3 per path + spare
+    // segments) and its tables (the kernels keep less)
     const uint64_t positions = 3 * r.n_paths + 64 * (2 + std::max<uint64_t>(r.n_threads, 1)) + 64;
     return positions * 8 + positions / 32 * 4 + positions / 64 * (18 + 1 + 8) + r.n_paths * 16 + partials;
   }
