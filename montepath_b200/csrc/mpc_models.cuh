@@ -602,9 +602,11 @@ __device__ __forceinline__ uint32_t poisson_tail(double u, double mean, double p
 // time; every thread of a request runs the same sequence, so the staged Sobol
 // source stays in lockstep.  FP64 keeps the reference's two-rounding products
 // and left-to-right sums.  The weights come in the path's precision (one
-// 16-byte load an op), the op counts by step instead of an event bit each, and
-// the samples by quads: 123 instructions a step in FP32, which alone is bound by
-// latency (60 us for 100,000 x 64, as before) and beside other groups by issue.
+// 16-byte load an op) with the number of steps after the op in the fourth word,
+// and the samples by quads.  Bound by latency (stack, weights and table loads at
+// 5 warps per scheduler: 100,000 x 64 in FP32 62.2 us with the op counts in a
+// table by step, a second load before each op, 57.8 so; the weights loaded one op
+// ahead spilled at 64 registers: 76).
 template <class Real, class Src>
 struct BridgeWalk {
   static_assert(kQuadSource<Src>, "bridge paths are drawn from scrambled Sobol");
@@ -638,22 +640,29 @@ struct BridgeWalk {
     w_left = (Real)0;
     op = 0;
   }
-  // The increment of step s (the host checked the program: it never needs
-  // more than kBridgeDepth values).
-  __device__ __forceinline__ Real next(const DevReq& q, Src& src, uint32_t s) {
-    for (uint32_t left = __ldg(q.bridge_counts + s); left > 0; --left, ++op) {
+  // The next op; returns the steps after it (the host checked the program: it
+  // never needs more than kBridgeDepth values).
+  __device__ __forceinline__ uint32_t midpoint(const DevReq& q, Src& src) {
+    uint32_t steps;
+    if constexpr (sizeof(Real) == 8) {
+      const double2* o = static_cast<const double2*>(q.bridge_ops) + 2 * op;
+      const double2 w = __ldg(o), d = __ldg(o + 1);
       const Real z = draw(src);
       stack[sp++] = top;
-      if constexpr (sizeof(Real) == 8) {
-        const double2* o = static_cast<const double2*>(q.bridge_ops) + 2 * op;
-        const double2 w = __ldg(o);
-        const double sd = __ldg(reinterpret_cast<const double*>(o + 1));
-        top = __dadd_rn(__dadd_rn(__dmul_rn(w.x, w_left), __dmul_rn(w.y, top)), __dmul_rn(sd, z));
-      } else {
-        const float4 o = __ldg(static_cast<const float4*>(q.bridge_ops) + op);
-        top = o.x * w_left + o.y * top + o.z * z;
-      }
+      top = __dadd_rn(__dadd_rn(__dmul_rn(w.x, w_left), __dmul_rn(w.y, top)), __dmul_rn(d.x, z));
+      steps = (uint32_t)d.y;
+    } else {
+      const float4 o = __ldg(static_cast<const float4*>(q.bridge_ops) + op);
+      const Real z = draw(src);
+      stack[sp++] = top;
+      top = o.x * w_left + o.y * top + o.z * z;
+      steps = (uint32_t)o.w;
     }
+    ++op;
+    return steps;
+  }
+  // The next step's increment.
+  __device__ __forceinline__ Real step(const DevReq& q) {
     Real inc;
     if constexpr (sizeof(Real) == 8)
       inc = __dmul_rn(__dsub_rn(top, w_left), q.bridge_inv_sqrt_dt);
@@ -710,7 +719,13 @@ __device__ __forceinline__ void unit_gbm_step(const DevReq& q, Src& src, double&
   if constexpr (BRIDGE) {  // increments from the Brownian bridge over the inputs
     BridgeWalk<Real, Src> bw;
     bw.begin(q, src);
-    for (; s < n; ++s) advance(bw.next(q, src, s));
+    uint32_t steps = n == 1 ? 1u : 0u;  // a longer path starts with an op
+    for (;;) {
+      for (; steps > 0; --steps) advance(bw.step(q));
+      if (++s >= n) break;  // n - 1 ops in all
+      steps = bw.midpoint(q, src);
+    }
+    s = n;
   } else if constexpr (kQuadSource<Src>) {
     for (; s + 4 <= n; s += 4) {  // four steps per quad of dimensions
       src.at_step(s, 4);

@@ -353,21 +353,20 @@ static int sampler_of(int sampling) {
 // BrownianBridgePlan::new (cpu.rs:5923-5962) flattened into the program the
 // device walks: the reference's interval stack is replayed; every pop is an op
 // (a midpoint of an interval longer than one step, consuming the next input
-// dimension) or a step, and a step records how many ops came before it since
-// the last one.  Ops carry the reference's weights and stddev, computed the same
+// dimension) or a step, and an op records how many steps come after it before
+// the next one.  Ops carry the reference's weights and stddev, computed the same
 // way.  Returns false if the walk would need a deeper stack than the device holds.
 static bool build_bridge_program(Prepared* p, uint32_t n, double maturity) {
   const double dt = maturity / double(n);
   p->bridge_ops.clear();
-  p->bridge_counts.clear();
   std::vector<std::pair<uint32_t, uint32_t>> intervals{{0u, n}};
-  uint32_t ops = 0, depth = 1, max_depth = 1;  // depth: values on the device stack (starts with W(T))
+  uint32_t steps = 0, depth = 1, max_depth = 1;  // depth: values on the device stack (starts with W(T))
   while (!intervals.empty()) {
     const auto [left, right] = intervals.back();
     intervals.pop_back();
     if (right <= left + 1) {  // a step: pops one value
-      p->bridge_counts.push_back(uint8_t(ops));
-      ops = 0;
+      if (!p->bridge_ops.empty()) p->bridge_ops.back() += 1.0;  // none before: the one step of a one-step path
+      ++steps;
       --depth;
       continue;
     }
@@ -378,14 +377,13 @@ static bool build_bridge_program(Prepared* p, uint32_t n, double maturity) {
     p->bridge_ops.push_back((t_mid - t_left) / denom);
     p->bridge_ops.push_back(std::sqrt((t_mid - t_left) * (t_right - t_mid) / denom));
     p->bridge_ops.push_back(0.0);
-    ++ops;
     max_depth = std::max(max_depth, ++depth);  // op: pushes the midpoint
     intervals.push_back({mid, right});
     intervals.push_back({left, mid});
   }
   p->q.bridge_sqrt_t = std::sqrt(maturity);
   p->q.bridge_inv_sqrt_dt = 1.0 / std::sqrt(dt);
-  return p->bridge_counts.size() == n && depth == 0 && max_depth <= kBridgeDepth && p->bridge_ops.size() == 4ull * (n - 1);
+  return steps == n && depth == 0 && max_depth <= kBridgeDepth && p->bridge_ops.size() == 4ull * (n - 1);
 }
 
 static std::vector<uint32_t> first_primes(size_t n) {
@@ -698,7 +696,7 @@ static int upload_aux(mpc_context* ctx, std::vector<Prepared*>& reqs) {
   for (Prepared* p : reqs) {
     bytes += p->halton.size() * sizeof(HaltonDim) + p->halton_weights.size() * 8 + 32;
     bytes += p->lhs.size() * sizeof(LhsDim) + 16;
-    bytes += p->bridge_ops.size() * 8 + p->bridge_counts.size() + 32;
+    bytes += p->bridge_ops.size() * 8 + 32;
     any = any || !p->halton.empty() || !p->lhs.empty() || p->q.bridge;
   }
   if (!any) return MPC_OK;
@@ -734,7 +732,6 @@ static int upload_aux(mpc_context* ctx, std::vector<Prepared*>& reqs) {
         for (size_t i = 0; i < p->bridge_ops.size(); ++i) out[i] = float(p->bridge_ops[i]);
         p->q.bridge_ops = static_cast<uint8_t*>(d_aux) + at;
       }
-      p->q.bridge_counts = static_cast<const uint8_t*>(place(p->bridge_counts.data(), p->bridge_counts.size()));
     }
   }
   MPC_CUDA(ctx, cudaMemcpyAsync(d_aux, host, off, cudaMemcpyHostToDevice, ctx->stream));

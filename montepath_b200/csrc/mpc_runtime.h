@@ -43,7 +43,6 @@ struct Prepared {
   std::vector<double> halton_weights;
   std::vector<LhsDim> lhs;
   std::vector<double> bridge_ops;       // [n_steps - 1][4]
-  std::vector<uint8_t> bridge_counts;   // [n_steps]
   uint64_t path_steps = 0;
 };
 

@@ -122,10 +122,9 @@ struct alignas(16) DevReq {
   uint64_t coarse_steps;
   double f_drift, f_vol, c_drift, c_vol, inv_sqrt_m, inv_fine, inv_coarse;
   // Brownian-bridge path construction (GBM stepwise with bridge Sobol), in the
-  // reference's depth-first order: step s is preceded by bridge_counts[s] ops
-  // (midpoints of longer intervals, each taking the next input dimension).
-  const void* bridge_ops;         // [n_steps - 1][4]: left weight, right weight, stddev, - (double, or float in FP32)
-  const uint8_t* bridge_counts;   // [n_steps]
+  // reference's depth-first order: ops (midpoints of longer
+  // intervals, each taking the next input dimension) with the steps after each.
+  const void* bridge_ops;         // [n_steps - 1][4]: left weight, right weight, stddev, steps after it (double, or float in FP32)
   double bridge_sqrt_t, bridge_inv_sqrt_dt;
   uint32_t bridge;                // 1: normals come through the bridge
   uint32_t n_scen;                // scenario kernel: legs (0 elsewhere)
