@@ -252,8 +252,8 @@ __device__ __forceinline__ float counter_normal_f32(uint32_t seed, uint32_t path
 __device__ __forceinline__ float counter_open01_fast(uint32_t h) {
   return h == 0xFFFFFFFFu ? 1.0f : __uint2float_rn(h + 1u) * 2.3283064365386963e-10f;
 }
-// Hardware approximations without the denormal scaling of the CUDA functions
-// built on them (the operands here are never denormal): the same values.
+// PTX's approximate base-2 logarithm, reciprocal and square root, flushing
+// denormals: the operands here are uniforms above 2^-54 and values of order one.
 __device__ __forceinline__ float log2_ftz(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

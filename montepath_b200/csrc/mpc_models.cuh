@@ -555,15 +555,10 @@ __device__ __forceinline__ Real normal(Src& s, uint32_t d) {
 
 template <class Real>
 __device__ __forceinline__ Real ex(Real x) {
-  if constexpr (sizeof(Real) == 4) {
-    // __expf without its denormal scaling (prices and discounted payoffs are
-    // far from it): the same value for every normal result
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
-    return y;
-  } else {
+  if constexpr (sizeof(Real) == 4)
+    return __expf(x);
+  else
     return exp(x);
-  }
 }
 __device__ __forceinline__ float sqrt_approx(float x) {
   float y;
