@@ -409,21 +409,27 @@ __device__ __forceinline__ double sobol_unit_f64(uint32_t x) {
   return ((double)(x >> 9) + 0.5) * 1.1920928955078125e-07;
 }
 
-// 1 / x to an ulp or two by Newton's iteration from the hardware's 20-bit
-// approximation, for normal x away from the range's ends.
+// 1 / x by Newton's iteration from the hardware's 20-bit approximation, for
+// normal x away from the range's ends: the first step leaves 2^-40, the second
+// squares that and rounds once, within 2^-27 units of half a unit in the last
+// place.
 __device__ __forceinline__ double newton_reciprocal(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   y = fma(y, fma(-x, y, 1.0), y);
   return fma(y, fma(-x, y, 1.0), y);
 }
-// num / den by the reciprocal and one correction with the exact remainder
-// (Markstein 1990): within a hair of half an ulp, without the tests and the
-// branch a general quotient needs.
-__device__ __forceinline__ double quotient(double num, double den) {
-  const double y = newton_reciprocal(den), q = num * y;
+// num / den by the reciprocal y = newton_reciprocal(den) and one correction with
+// the exact remainder (Markstein 1990), without the tests and the branch a
+// general quotient needs, for quotients and remainders in the normal range.  It
+// differs from the correctly rounded quotient only where the exact one lies
+// within about 2^-50 units of a rounding boundary (tests/test_gpu_arithmetic.py
+// finds none in 2^23 arguments of the inverse normal and 10^6 normal equations).
+__device__ __forceinline__ double quotient(double num, double den, double y) {
+  const double q = num * y;
   return fma(fma(-den, q, num), y, q);
 }
+__device__ __forceinline__ double quotient(double num, double den) { return quotient(num, den, newton_reciprocal(den)); }
 
 // ------------------------------------------------------- Acklam inverse ---
 // inverse_standard_normal (cpu.rs:6012-6061): the reference rational in FP64.
@@ -603,6 +609,77 @@ __device__ __forceinline__ double lhs_place(const LhsDim* __restrict__ dim, uint
     stratum = (double)((a.x * point + a.y) % n_paths);
   }
   return stratum + open01_from_u64(splitmix64(b.x ^ mixed));
+}
+
+// ----------------------------------------- Longstaff-Schwartz arithmetic ---
+// x / 6 as x C + x c, C = 1/6 rounded and c the rest of 1/6: one multiplication
+// and one FMA (division by a constant known in advance, Brisebarre, Muller and
+// Raina 2004).  In FP32 this is the correctly rounded quotient (checked for
+// every mantissa); in FP64 it is within an ulp of it.
+__device__ __forceinline__ float sixth(float x) { return fmaf(x, 0.16666667f, x * -4.967053731882189e-09f); }
+__device__ __forceinline__ double sixth(double x) {
+  return fma(x, 0.16666666666666666, x * 9.25185853854297e-18);
+}
+
+template <class Real>
+__device__ __forceinline__ void laguerre4(Real x, Real b[4]) {
+  // laguerre_lsm_basis (cpu.rs:7667-7682); degrees above `degree` are unused
+  const Real x2 = x * x, x3 = x2 * x;
+  b[0] = (Real)1;
+  b[1] = (Real)1 - x;
+  b[2] = (Real)1 - (Real)2 * x + (Real)0.5 * x2;
+  b[3] = (Real)1 - (Real)3 * x + (Real)1.5 * x2 - sixth(x3);
+}
+
+// solve_lsm_normal_equations (cpu.rs:7684-7736) for a compile-time size:
+// Gauss-Jordan with partial pivoting in FP64, the reference's operations in
+// its order, every index static (the pivot row swap is a predicated exchange),
+// so the system stays in registers.  FP64 paths divide each entry of a pivot row
+// by the pivot (|pivot| > 1e-12), all from one reciprocal; RECIP (FP32 paths)
+// multiplies by the reciprocal.
+template <int DIM, bool RECIP>
+__device__ __forceinline__ bool solve_fixed(double a[4][4], double rhs[4]) {
+#pragma unroll
+  for (int piv = 0; piv < DIM; ++piv) {
+    int best = piv;
+    double best_abs = fabs(a[piv][piv]);
+#pragma unroll
+    for (int row = piv + 1; row < DIM; ++row) {
+      const double c = fabs(a[row][piv]);
+      if (c > best_abs) {
+        best = row;
+        best_abs = c;
+      }
+    }
+    if (best_abs <= 1e-12) return false;
+#pragma unroll
+    for (int row = piv + 1; row < DIM; ++row) {
+      if (row == best) {
+#pragma unroll
+        for (int c = piv; c < DIM; ++c) {
+          const double t = a[piv][c];
+          a[piv][c] = a[row][c];
+          a[row][c] = t;
+        }
+        const double t = rhs[piv];
+        rhs[piv] = rhs[row];
+        rhs[row] = t;
+      }
+    }
+    const double pv = a[piv][piv], ip = newton_reciprocal(pv);
+#pragma unroll
+    for (int c = piv + 1; c < DIM; ++c) a[piv][c] = RECIP ? a[piv][c] * ip : quotient(a[piv][c], pv, ip);
+    rhs[piv] = RECIP ? rhs[piv] * ip : quotient(rhs[piv], pv, ip);
+#pragma unroll
+    for (int row = 0; row < DIM; ++row) {
+      if (row == piv) continue;
+      const double f = a[row][piv];
+#pragma unroll
+      for (int c = piv + 1; c < DIM; ++c) a[row][c] -= f * a[piv][c];
+      rhs[row] -= f * rhs[piv];
+    }
+  }
+  return true;
 }
 
 // ------------------------------------------------------------- reductions -

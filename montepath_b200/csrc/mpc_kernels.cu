@@ -1162,76 +1162,6 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-// x / 6 as x C + x c, C = 1/6 rounded and c the rest of 1/6: one multiplication
-// and one FMA (division by a constant known in advance, Brisebarre, Muller and
-// Raina 2004).  In FP32 this is the correctly rounded quotient (checked for
-// every mantissa); in FP64 it is within an ulp of it.
-__device__ __forceinline__ float sixth(float x) { return fmaf(x, 0.16666667f, x * -4.967053731882189e-09f); }
-__device__ __forceinline__ double sixth(double x) {
-  return fma(x, 0.16666666666666666, x * 9.25185853854297e-18);
-}
-
-template <class Real>
-__device__ __forceinline__ void laguerre4(Real x, Real b[4]) {
-  // laguerre_lsm_basis (cpu.rs:7667-7682); degrees above `degree` are unused
-  const Real x2 = x * x, x3 = x2 * x;
-  b[0] = (Real)1;
-  b[1] = (Real)1 - x;
-  b[2] = (Real)1 - (Real)2 * x + (Real)0.5 * x2;
-  b[3] = (Real)1 - (Real)3 * x + (Real)1.5 * x2 - sixth(x3);
-}
-
-// solve_lsm_normal_equations (cpu.rs:7684-7736) for a compile-time size:
-// Gauss-Jordan with partial pivoting in FP64, the reference's operations in
-// its order but with each pivot row scaled by the pivot's reciprocal
-// (|pivot| > 1e-12), every
-// index static (the pivot row swap is a predicated exchange), so the system
-// stays in registers.
-template <int DIM>
-__device__ __forceinline__ bool solve_fixed(double a[4][4], double rhs[4]) {
-#pragma unroll
-  for (int piv = 0; piv < DIM; ++piv) {
-    int best = piv;
-    double best_abs = fabs(a[piv][piv]);
-#pragma unroll
-    for (int row = piv + 1; row < DIM; ++row) {
-      const double c = fabs(a[row][piv]);
-      if (c > best_abs) {
-        best = row;
-        best_abs = c;
-      }
-    }
-    if (best_abs <= 1e-12) return false;
-#pragma unroll
-    for (int row = piv + 1; row < DIM; ++row) {
-      if (row == best) {
-#pragma unroll
-        for (int c = piv; c < DIM; ++c) {
-          const double t = a[piv][c];
-          a[piv][c] = a[row][c];
-          a[row][c] = t;
-        }
-        const double t = rhs[piv];
-        rhs[piv] = rhs[row];
-        rhs[row] = t;
-      }
-    }
-    const double ip = newton_reciprocal(a[piv][piv]);
-#pragma unroll
-    for (int c = piv + 1; c < DIM; ++c) a[piv][c] *= ip;
-    rhs[piv] *= ip;
-#pragma unroll
-    for (int row = 0; row < DIM; ++row) {
-      if (row == piv) continue;
-      const double f = a[row][piv];
-#pragma unroll
-      for (int c = piv + 1; c < DIM; ++c) a[row][c] -= f * a[piv][c];
-      rhs[row] -= f * rhs[piv];
-    }
-  }
-  return true;
-}
-
 constexpr int kLsmBlock = (int)kLsmThreads;
 
 constexpr int kLsmMaxP = (int)kLsmPathsPerThreadMax;
@@ -1317,6 +1247,7 @@ __device__ __forceinline__ double sum_warps16(const double* rows, uint32_t mom) 
   return e + o;
 }
 // s_bad: shared flag, 0 until a wait fails (then the job's blocks all leave).
+template <bool RECIP>
 __device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, uint32_t round, int coeffs,
                                                  double* fold, double* s_mom, double* s_beta, int* s_ok, int* s_bad) {
   const uint64_t base_at = (uint64_t)round * nb * 16;
@@ -1382,7 +1313,12 @@ __device__ __forceinline__ bool lsm_gather_solve(const LsmArgs& a, uint32_t nb, 
     for (int r = 0; r < 4; ++r) atb[r] = s_mom[10 + r];
     // rows and columns past the basis degree are never read
     int ok = s_mom[14] >= (double)coeffs ? 1 : 0;
-    if (ok) ok = (coeffs == 2 ? solve_fixed<2>(ata, atb) : coeffs == 3 ? solve_fixed<3>(ata, atb) : solve_fixed<4>(ata, atb)) ? 1 : 0;
+    if (ok)
+      ok = (coeffs == 2   ? solve_fixed<2, RECIP>(ata, atb)
+            : coeffs == 3 ? solve_fixed<3, RECIP>(ata, atb)
+                          : solve_fixed<4, RECIP>(ata, atb))
+               ? 1
+               : 0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) s_beta[r] = (ok && r < coeffs) ? atb[r] : 0.0;
     *s_ok = ok;
@@ -1568,7 +1504,7 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(const LsmArgs* __rest
     if (si > 0) load_date(si - 1);  // next date's values, in flight during the wait
     // Every block waits (bounded) for all blocks' partials of this date, then
     // sums them in block order and solves the normal equations itself.
-    if (!lsm_gather_solve(a, nb, round++, coeffs, s_fold, s_mom, s_beta, &s_ok, &s_bad)) return;
+    if (!lsm_gather_solve<sizeof(Real) == 4>(a, nb, round++, coeffs, s_fold, s_mom, s_beta, &s_ok, &s_bad)) return;
     if (s_ok) {
       ++regressions;
       const Real b0 = (Real)s_beta[0], b1 = (Real)s_beta[1], b2 = (Real)s_beta[2], b3 = (Real)s_beta[3];
