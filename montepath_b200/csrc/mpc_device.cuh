@@ -612,13 +612,15 @@ __device__ __forceinline__ double lhs_place(const LhsDim* __restrict__ dim, uint
 }
 
 // ----------------------------------------- Longstaff-Schwartz arithmetic ---
-// x / 6 as x C + x c, C = 1/6 rounded and c the rest of 1/6: one multiplication
-// and one FMA (division by a constant known in advance, Brisebarre, Muller and
-// Raina 2004).  In FP32 this is the correctly rounded quotient (checked for
-// every mantissa); in FP64 it is within an ulp of it.
+// x / 6.  FP32: x C + x c with C = 1/6 rounded and c the rest of it, one
+// multiplication and one FMA (division by a constant known in advance,
+// Brisebarre, Muller and Raina 2004).  FP64: x C, less than one unit in the last
+// place off, corrected by its exact remainder (Markstein 1990).  Both are the
+// correctly rounded quotient (tests/test_gpu_arithmetic.py: every FP32 mantissa).
 __device__ __forceinline__ float sixth(float x) { return fmaf(x, 0.16666667f, x * -4.967053731882189e-09f); }
 __device__ __forceinline__ double sixth(double x) {
-  return fma(x, 0.16666666666666666, x * 9.25185853854297e-18);
+  const double c = 0.16666666666666666, q = x * c;
+  return fma(fma(-6.0, q, x), c, q);
 }
 
 template <class Real>

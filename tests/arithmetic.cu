@@ -31,6 +31,20 @@ __global__ void quotient_kernel(const double* num, const double* den, uint64_t n
   plain_inv[i] = __drcp_rn(den[i]);
 }
 
+__global__ void sixth_f32_kernel(uint32_t first, uint32_t n, unsigned long long* differing) {
+  const uint64_t i = thread_index();
+  if (i >= n) return;
+  const float x = __uint_as_float(first + (uint32_t)i);
+  if (__float_as_uint(sixth(x)) != __float_as_uint(__fdiv_rn(x, 6.0f))) atomicAdd(differing, 1ull);
+}
+
+__global__ void sixth_f64_kernel(const double* x, uint64_t n, double* ours, double* plain) {
+  const uint64_t i = thread_index();
+  if (i >= n) return;
+  ours[i] = sixth(x[i]);
+  plain[i] = __ddiv_rn(x[i], 6.0);
+}
+
 // solve_lsm_normal_equations with every division CUDA's.
 template <int DIM>
 __device__ bool solve_plain(double a[4][4], double rhs[4]) {
@@ -96,6 +110,24 @@ extern "C" int quotients(const double* num, const double* den, uint64_t n, doubl
   cudaMemcpy(plain, bp.p, n * 8, cudaMemcpyDeviceToHost);
   cudaMemcpy(ours_inv, boi.p, n * 8, cudaMemcpyDeviceToHost);
   cudaMemcpy(plain_inv, bpi.p, n * 8, cudaMemcpyDeviceToHost);
+  return finish();
+}
+
+// Floats with the bit patterns first .. first + n - 1: how many differ.
+extern "C" int sixths_f32(uint32_t first, uint32_t n, unsigned long long* differing) {
+  Buffer count(8);
+  cudaMemset(count.p, 0, 8);
+  sixth_f32_kernel<<<blocks(n), 256>>>(first, n, count.as<unsigned long long>());
+  cudaMemcpy(differing, count.p, 8, cudaMemcpyDeviceToHost);
+  return finish();
+}
+
+extern "C" int sixths_f64(const double* x, uint64_t n, double* ours, double* plain) {
+  Buffer bx(n * 8), bo(n * 8), bp(n * 8);
+  cudaMemcpy(bx.p, x, n * 8, cudaMemcpyHostToDevice);
+  sixth_f64_kernel<<<blocks(n), 256>>>(bx.as<double>(), n, bo.as<double>(), bp.as<double>());
+  cudaMemcpy(ours, bo.p, n * 8, cudaMemcpyDeviceToHost);
+  cudaMemcpy(plain, bp.p, n * 8, cudaMemcpyDeviceToHost);
   return finish();
 }
 

@@ -64,6 +64,18 @@ def test_inverse_normal_quotients(lib):
     same_quotients(lib, *centre_rational(np.random.default_rng(5).uniform(0.02425, 0.97575, 1 << 22)))
 
 
+def test_sixths(lib):
+    n = ctypes.c_ulonglong()
+    for exponent in (-40, -20, -1, 0, 1, 20):  # all 2^23 mantissas
+        assert lib.sixths_f32(ctypes.c_uint32((exponent + 127) << 23), ctypes.c_uint32(1 << 23), ctypes.byref(n)) == 0
+        assert n.value == 0
+    rng = np.random.default_rng(7)
+    x = rng.uniform(1.0, 2.0, 1 << 22) * np.exp2(rng.integers(-60, 20, 1 << 22))
+    ours, plain = np.zeros_like(x), np.zeros_like(x)
+    assert lib.sixths_f64(p(x), ctypes.c_uint64(x.size), p(ours), p(plain)) == 0
+    assert np.array_equal(ours, plain), int((ours != plain).sum())
+
+
 @pytest.mark.parametrize("dim", [2, 3, 4])
 def test_lsm_normal_equations(lib, dim):
     """Regressions of a date with `dim` to 300 in-the-money paths: prices spread
