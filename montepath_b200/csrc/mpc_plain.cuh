@@ -37,8 +37,10 @@ struct PlainSource<SMP_XORSHIFT> {
   using type = XorshiftPairs<double>;
 };
 
-// Resident blocks the register allocation must allow: a basket keeps its
-// Cholesky factor and per-asset constants in registers.
+// Resident blocks the register allocation must allow.  A basket keeps the FP64
+// sums of up to 8 assets beside a sample in the making: 64 registers (8 blocks)
+// spill, 2,000 x 252 of 8 assets 397 -> 419 us pseudorandom and 601 -> 642 on the
+// counter hash, where larger requests gain 2 to 8%.
 constexpr int plain_min_blocks(int fam) { return fam == FAM_BASKET ? 3 : 8; }
 
 // The block's moment sums as its tile partial; the request's last tile to

@@ -102,3 +102,12 @@ def test_halton_wide_digit_products(backend):
     a = backend.price(make_request("european_call", dict(kw, precision="fp32_path")))
     b = backend.price(make_request("european_call", dict(kw, precision="fp64_plain")))
     assert abs(a.price - b.price) < 0.01 * b.stderr, (a.price, b.price, b.stderr)
+
+
+@pytest.mark.parametrize("assets", [1, 2, 5, 8])
+@pytest.mark.parametrize("sampling", ["randomized_halton", "latin_hypercube"])
+def test_plain_lattice_baskets(backend, assets, sampling):
+    """A step's normals drawn in a loop (one asset: without it)."""
+
+    check(backend, "basket_call", method="stepwise", spots=[100.0] * assets, sigmas=[0.2] * assets,
+          weights=[1.0 / assets] * assets, corr=0.3, n_paths=1003, n_steps=7, seed=5, sampling=sampling)
