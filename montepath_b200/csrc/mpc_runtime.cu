@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -90,14 +91,27 @@ int scratch(mpc_context* ctx, const std::string& name, size_t bytes, void** out)
   return MPC_OK;
 }
 
-// Refuses a request whose documented size alone passes the context's budget.
-// The kernels keep less on the device than mpc_estimate_bytes states, but a
-// request beyond the budget stays refused.
-static int within_budget(mpc_context* ctx, const char* name, uint64_t bytes) {
-  if (bytes <= ctx->budget) return MPC_OK;
+// Admission of the FP64 paths.  Their documented sizes count samples, payoffs and
+// tables as buffers in device memory; the kernels keep less, but what those
+// buffers do not fit beside the context's other ones stays refused.  `sizes`: the
+// documented buffers; `own`: the buffers that hold their place now.
+static int within_budget(mpc_context* ctx, const char* name, std::initializer_list<uint64_t> sizes,
+                         std::initializer_list<const char*> own) {
+  uint64_t total = ctx->live_bytes;
+  for (const char* b : own) {
+    auto it = ctx->bufs.find(b);
+    if (it != ctx->bufs.end()) total -= it->second.bytes;
+  }
+  for (uint64_t s : sizes) total += (std::max<uint64_t>(s, 16) + 255) & ~uint64_t(255);
+  if (total <= ctx->budget) return MPC_OK;
   return fail(ctx, MPC_E_OOM_BUDGET,
-              "request needs " + std::to_string(bytes) + " device bytes for '" + name +
+              "request needs " + std::to_string(total) + " device bytes with '" + name +
                   "', beyond the HBM budget of " + std::to_string(ctx->budget) + " bytes");
+}
+// Their buffers for the reduction: descriptor, partials of 2,048 units, moments, counter.
+static uint64_t documented_reduction_bytes(uint64_t units) {
+  auto align = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
+  return align(sizeof(DevReq)) + align((units + 2047) / 2048 * MPC_MOMENTS * sizeof(double)) + 2 * 256;
 }
 
 static int grow_pinned(mpc_context* ctx, void** area, size_t* held, size_t bytes, void** out) {
@@ -976,8 +990,11 @@ static int run_plain(mpc_context* ctx, Prepared* p, mpc_result_t* out, double* p
   if (st != MPC_OK) return st;
   DevReq& q = p->q;
   const uint64_t units = q.n_units;
-  // the request's documented size counts every sample
-  if ((st = within_budget(ctx, "plain samples", units * q.normals_per_unit * sizeof(double)))) return st;
+  if ((st = within_budget(ctx, "plain samples",
+                          {units * q.normals_per_unit * sizeof(double), units * sizeof(double),
+                           q.cv ? units * sizeof(double) : 0, documented_reduction_bytes(units)},
+                          {"plain_pay", "plain_part", "plain_done"})))
+    return st;
   const uint32_t lanes = plain_lanes(*p);
   const uint32_t block = lanes > 1 ? 128u : plain_block(units);
   // units per thread: 1, or up to 4 for units of a few samples, while the
@@ -1055,8 +1072,14 @@ static int run_merton_stream(mpc_context* ctx, Prepared* p, mpc_result_t* out, d
   const uint64_t blocks = uint64_t(a.blocks_per_chunk) * a.n_chunks;
   if (blocks > 0x7FFFFFFFull) return fail(ctx, MPC_E_UNSUPPORTED, "too many stream blocks for one launch");
   int st;
-  // the request's documented size counts one 8-byte word per stream position
-  if ((st = within_budget(ctx, "merton stream", a.n_chunks * (3 * max_chunk + 8) * 8))) return st;
+  {  // documented: stream outputs, jump bits, maps of 64-position segments and their states, path starts, payoffs
+    const uint64_t segs = (3 * max_chunk + 8 + 63) / 64, padded = a.n_chunks * (segs + 1) * 64;
+    if ((st = within_budget(ctx, "merton stream",
+                            {padded * 8, padded / 32 * 4, a.n_chunks * segs * 18, a.n_chunks * segs,
+                             a.n_chunks * segs * 8, a.mean != 0.0 ? n * 8 : 0, n * 8, documented_reduction_bytes(n)},
+                            {"merton_ws", "merton_done", "plain_pay"})))
+      return st;
+  }
   // run entries | block maps | halo | blocks' path counts | partials | block states
   const size_t o_map = blocks * kMertonThreads * 4, o_halo = o_map + blocks * 32, o_before = o_halo + blocks * 32,
                o_part = o_before + blocks * 8, o_state = o_part + blocks * 16, ws_bytes = o_state + blocks * 4;

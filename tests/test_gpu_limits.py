@@ -29,3 +29,31 @@ def test_prices_below_the_fp32_normal_range(backend, workload, kw, sampling):
     want = backend.price(make_request(workload, dict(cfg, precision="fp64_plain"))).price
     got = backend.price(make_request(workload, cfg)).price
     assert abs(got - want) <= 1e-4 * want, (got, want)
+
+
+MILLION = 1_000_000
+
+
+@pytest.mark.parametrize("workload,kw,refused,accepted", [
+    # samples and half the payoffs; samples and payoffs
+    ("european_call", dict(method="stepwise"), 8 * 16 + 4, 8 * 16 + 8),
+    # samples, payoffs and half the control values; all of them
+    ("european_call", dict(method="stepwise", technique="control_variate"), 8 * 16 + 12, 8 * 16 + 16),
+    # three stream positions, their bits and maps, path starts and half the payoffs; all of them
+    ("european_call", dict(model="merton", method="terminal"), 26 + 8 + 4, 26 + 8 + 8),
+])
+def test_budget_counts_every_documented_buffer(workload, kw, refused, accepted):
+    """FP64 admission by the documented sizes (bytes per path): the kernels keep
+    less in device memory, but the budget a request needs has not changed."""
+
+    from montepath_b200 import abi
+    from montepath_b200.backend import BackendError, CudaBackend
+
+    r = make_request(workload, dict(kw, n_paths=MILLION, n_steps=16, sampling="pseudorandom", precision="fp64_plain"))
+    with CudaBackend(0, hbm_budget_bytes=refused * MILLION) as small:
+        with pytest.raises(BackendError) as err:
+            small.price(r)
+        assert err.value.status == abi.E_OOM_BUDGET
+    with CudaBackend(0, hbm_budget_bytes=accepted * MILLION + (2 << 20)) as enough:  # and the context's own tables
+        assert enough.price(r).price > 0.0
+        assert enough.price(r).price > 0.0  # beside the buffers of the first call
