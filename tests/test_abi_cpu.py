@@ -314,3 +314,17 @@ def test_serving_command_line_help():
     with pytest.raises(SystemExit) as done:
         serving.main(["--help"])
     assert done.value.code == 0
+
+
+@pytest.mark.parametrize("workload", ["european_call", "down_and_out_call"])
+@pytest.mark.parametrize("precision", ["fp32_path", "fp64_plain"])
+def test_cost_estimates_off_their_measured_cell_are_derived(workload, precision):
+    """Stepwise GBM on Sobol is estimated away from its measured rate, so that it
+    must not be called measured; the same request on another stream is."""
+
+    from montepath_b200 import production
+
+    cfg = {"n_paths": 1 << 20, "n_steps": 64, "method": "stepwise", "precision": precision}
+    cost = production.estimate_cost(workload, dict(cfg, sampling="scrambled_sobol"))
+    assert cost["confidence"] == "derived"
+    assert production.estimate_cost(workload, dict(cfg, sampling="pseudorandom"))["confidence"] == "measured"
