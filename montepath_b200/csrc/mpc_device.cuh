@@ -17,10 +17,6 @@ namespace mpc {
 // T^(2^b) for b = 0..63 in nibble form: jump[b][q][v] = T^(2^b) applied to
 // the nibble value v placed at bit position 4q.  Jumping k draws ahead costs
 // popcount(k) * 16 table lookups.
-struct JumpTables {
-  const uint64_t* nibble;  // [64][16][16]
-};
-
 __device__ __forceinline__ uint64_t gf2_apply(const uint64_t* __restrict__ table, uint64_t x) {
   uint64_t y = 0;
 #pragma unroll
@@ -374,25 +370,6 @@ __device__ __forceinline__ uint32_t nested_uniform_scramble(uint32_t x, uint32_t
 }
 __host__ __device__ __forceinline__ uint32_t hash_combine(uint32_t seed, uint32_t v) {
   return seed ^ (v + 0x9e3779b9u + (seed << 6) + (seed >> 2));
-}
-__device__ __forceinline__ uint32_t sobol_product(const uint32_t* __restrict__ table_dim, uint32_t index) {
-  // table_dim: 8 x 16 words for this dimension (bit 0 of the index = MSB direction)
-  uint32_t x = 0;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) x ^= table_dim[q * 16 + ((index >> (4 * q)) & 0xFu)];
-  return x;
-}
-// Sobol sample of (point, normal_index) with the reference's block and
-// dimension-wrap seeding (ScrambledSobol::standard_normal, cpu.rs:5665-5677).
-__device__ __forceinline__ uint32_t sobol_point(const uint32_t* __restrict__ table, uint64_t point,
-                                                uint32_t normal_index, uint32_t seed32) {
-  uint32_t block = (uint32_t)(point >> 16);
-  uint32_t local = (uint32_t)(point & 0xFFFFu);
-  uint32_t dim = normal_index & (MPC_SOBOL_TABLE_DIMS - 1);
-  uint32_t seed = seed32 + (normal_index / MPC_SOBOL_TABLE_DIMS) + block * 0x9E3779B9u;
-  uint32_t shuffled = nested_uniform_scramble(local, seed);
-  uint32_t x = sobol_product(table + dim * 128, shuffled);
-  return nested_uniform_scramble(x, hash_combine(seed, dim));
 }
 // 23-bit midpoint uniform: exact in both precisions, never 0 or 1.
 __device__ __forceinline__ float sobol_unit_f32(uint32_t x) {

@@ -785,7 +785,7 @@ __device__ __forceinline__ void sum_rows(const double* rows, uint32_t n_rows, ui
 }
 
 // Next tile of a scenario launch, first the block's own index; the cursor is
-// q.tiles_done[1] and the last block to finish leaves both words zero.
+// q.tiles_done[1], and the last block to go leaves all three words zero.
 __device__ __forceinline__ uint32_t next_scenario_tile(const DevReq& q, uint32_t* s_tile) {
   if (threadIdx.x == 0) *s_tile = gridDim.x + atomicAdd(q.tiles_done + 1, 1u);
   __syncthreads();

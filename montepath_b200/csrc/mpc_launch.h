@@ -137,8 +137,8 @@ constexpr uint32_t kLsmThreads = 512;
 
 // Bump-and-revalue legs sharing every normal: one request q (GBM step,
 // GBM terminal or Heston; xorshift, Sobol or counter-hash samples; any
-// technique) and its legs' parameters; tiles_done[0] and [1] are zero before and
-// after; with NM =
+// technique) and its legs' parameters; q.tiles_done holds three words, zero
+// before and after (tiles done, cursor, blocks gone); with NM =
 // scenario_moments(technique), q.partials must hold [n_tiles][kMaxScen][NM]
 // doubles and q.moments [kMaxScen][NM]: sum p, sum p^2 (pair averages for
 // antithetic requests), then for control variates sum c, sum c^2, sum p c.

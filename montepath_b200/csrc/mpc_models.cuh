@@ -38,7 +38,7 @@ struct SrcCtx {
 // for every point of one aligned 4,096-point group, and the XOR of their five
 // nibble rows is one word per dimension.  The points a block runs together
 // (one iteration of a tile: at most 512 consecutive aligned units, the tile's
-// idle threads repeating the iteration's first unit) lie in one such group.
+// idle threads repeating its last unit) lie in one such group.
 // The output scramble's seed of a dimension, hash_combine(seed_g, dim),
 // depends on the block's seed and the dimension alone, so a last row holds
 // it for the window's dimensions: a quad reads its four seeds with one load.
@@ -50,27 +50,16 @@ constexpr uint32_t kSobolConstRow = kSobolLowRows;              // XOR of the up
 constexpr uint32_t kSobolSeedRow = kSobolLowRows + 1;           // output-scramble seed per dimension
 constexpr uint32_t kSobolWindowWords = (kSobolLowRows + 2) * kSobolRowStride;  // 13,600 bytes
 
-// Phi^-1(u) for a 23-bit midpoint uniform u from the segment table: v =
-// min(u, 1 - u) (exact) selects binade and one of 32 segments from its
-// exponent and top mantissa bits, the remaining 18 mantissa bits give the
-// position t in [0, 1/32) in the segment (they sit below 1.0's exponent as
-// they are, so no shift is needed), and the segment's cubic gives Phi^-1(v).
-// Defined for v in [2^-24, 1/2), which every 23-bit midpoint uniform meets.
-__device__ __forceinline__ float icdf_segments(const float4* __restrict__ seg, float u) {
-  const float v = fminf(u, 1.0f - u);
-  const uint32_t bits = __float_as_uint(v);
-  const uint32_t idx = (bits >> 18) - (103u << 5);  // (exponent - 103) * 32 + top 5 mantissa bits
-  const float t = __int_as_float((bits & 0x3FFFFu) | 0x3F800000u) - 1.0f;
-  const float4 c = seg[idx];
-  const float p = fmaf(fmaf(fmaf(c.w, t, c.z), t, c.y), t, c.x);
-  return u < 0.5f ? p : -p;
-}
-// icdf_segments(seg, sobol_unit_f32_bits(x)) from the Sobol sample's bits.
-// With m = x >> 9 the uniform is u = (m + 0.5) 2^-23, and its mirror 1 - u
-// is the same expression of the 23-bit complement of m, so
+// Phi^-1(u) for the 23-bit midpoint uniform u of a Sobol sample x, from the
+// segment table.  With m = x >> 9 the uniform is u = (m + 0.5) 2^-23, and its
+// mirror 1 - u is the same expression of the 23-bit complement of m, so
 // v = min(u, 1 - u) is built from x ^ (x >> 31, arithmetic): the complement
-// exactly when bit 31 (u > 1/2) is set, which also gives the result's sign.
-// Equal bit for bit to the two-step form, with no compare or select.
+// exactly when bit 31 (u > 1/2) is set, which also gives the result's sign, with
+// no compare or select.  v selects binade and one of 32 segments from its
+// exponent and top mantissa bits, the remaining 18 mantissa bits give the
+// position t in [0, 1/32) in the segment (they sit below 1.0's exponent as they
+// are, so no shift is needed), and the segment's cubic gives Phi^-1(v).
+// Defined for v in [2^-24, 1/2), which every 23-bit midpoint uniform meets.
 __device__ __forceinline__ float icdf_sobol_bits(const float4* __restrict__ seg, uint32_t x) {
   const uint32_t xm = x ^ (uint32_t)((int32_t)x >> 31);
   const float v = __fsub_rn(__uint_as_float((xm >> 9) + 0x3F800000u), 0.99999994f);
@@ -130,9 +119,10 @@ struct Source<SMP_COUNTER> {
 // Scrambled Sobol with the per-point work hoisted: the Owen-shuffled index
 // and its nibble offsets depend only on (point, dimension group of 256), so
 // they are recomputed when a path crosses into the next group; per
-// dimension only the 8 table lookups and the output scramble remain.  The
-// values equal sobol_point() bit for bit.  Reads the [dim][q][v] layout from
-// global memory (generators and the FP64 plain path).
+// dimension only the 8 table lookups and the output scramble remain.  Blocks of
+// 2^16 points and the dimension wrap are seeded as ScrambledSobol::
+// standard_normal does (cpu.rs:5665-5677).  Reads the [dim][q][v] layout from
+// global memory (the sample generator).
 template <>
 struct Source<SMP_SOBOL> {
   const uint32_t* table;
@@ -347,10 +337,6 @@ struct SobolQuad {
     return __brev(lk_permute(K == 0 ? x0 : K == 1 ? x1 : K == 2 ? x2 : x3, K == 0 ? s0 : K == 1 ? s1 : K == 2 ? s2 : s3));
   }
   template <int K>
-  __device__ __forceinline__ float take_u(uint32_t d0) const {
-    return sobol_unit_f32_bits(take<K>(d0));
-  }
-  template <int K>
   __device__ __forceinline__ float take_n(uint32_t d0) const {
     return icdf_sobol_bits(icdf, take<K>(d0));
   }
@@ -366,8 +352,6 @@ struct SobolQuad {
   }
   __device__ __forceinline__ float u32(uint32_t d) { return sobol_unit_f32_bits(sample(d)); }
   __device__ __forceinline__ float n32(uint32_t d) { return icdf_sobol_bits(icdf, sample(d)); }
-  __device__ __forceinline__ double u64(uint32_t d) { return sobol_unit_f64(sample(d)); }
-  __device__ __forceinline__ double n64(uint32_t d) { return icdf_f64(u64(d)); }
 };
 
 // The FP64 plain path's Sobol samples: the staged window, FP64 inverse normal.
@@ -483,7 +467,7 @@ struct XorshiftPairs {
   }
 };
 
-// Sources with the explicit-quad interface (quad_load / take_n / take_u).
+// Sources with the explicit-quad interface (quad_load / take_n).
 template <class S>
 constexpr bool kQuadSource = false;
 template <>
