@@ -68,15 +68,16 @@ struct LoopArgs {
 cudaError_t launch_serve_loop(const LoopArgs& a, const DeviceTables& tabs, int grid, cudaStream_t stream);
 int serve_loop_blocks_per_sm();
 
-// FP64 plain path: one launch per request (q.n_tiles blocks of `block`
-// threads, 32 to 128), moments written to q.moments by the last block;
-// *q.tiles_done is zero before and after.
-cudaError_t launch_plain(const DevReq& q, int sampler, const DeviceTables& tabs, int block, cudaStream_t stream);
+// FP64 plain path: one launch per request (q.n_tiles blocks of kPlainBlock
+// threads), moments written to q.moments by the last block; *q.tiles_done is
+// zero before and after.
+constexpr uint32_t kPlainBlock = 128;
+cudaError_t launch_plain(const DevReq& q, int sampler, const DeviceTables& tabs, cudaStream_t stream);
 // The same for pseudorandom stepwise GBM with `lanes` (2 to 32, a power of two)
-// threads per path, block = q.tile_units * lanes; each lane holds at most
+// threads per path, q.tile_units * lanes = kPlainBlock; each lane holds at most
 // kPlainSplitNormals normals.
 constexpr uint32_t kPlainSplitNormals = 32;
-cudaError_t launch_plain_split(const DevReq& q, const DeviceTables& tabs, int block, uint32_t lanes, cudaStream_t stream);
+cudaError_t launch_plain_split(const DevReq& q, const DeviceTables& tabs, uint32_t lanes, cudaStream_t stream);
 // Fills the MPC_ICDF_TAIL values of DeviceTables::icdf_tail.
 cudaError_t launch_icdf_tail(double* d_out, cudaStream_t stream);
 

@@ -1,9 +1,12 @@
 // mpc_plain.cuh -- the FP64 plain path: one request per launch, every sample
 // generated where it is used, stepped, paid and reduced in one kernel.
 //
-// One unit per thread, one tile per block; the hardware's block scheduler
-// balances the tiles, so small blocks (128 threads, fewer for small requests,
-// plain_block) keep the last wave full.  The descriptor travels as a kernel
+// One unit per thread (up to four for short units), one tile per block; the
+// hardware's block scheduler balances the tiles, so blocks of 128 threads keep the
+// last wave full.  Blocks of 64 and 32 are no faster for requests that leave SMs
+// without a block either, since every block stages its own tables: Heston x 64 on
+// Sobol 1,000 paths 41 / 43 / 45 us with 128 / 64 / 32 threads, 20,000 paths
+// 47 / 48 / 55; Asian x 64 on Halton 1,000 paths 58 / 62 / 70.  The descriptor travels as a kernel
 // parameter and the last tile writes the moments straight into the host's
 // pinned buffer: a request is one launch with no copies.  Before, samples
 // were written to HBM, read back by a second kernel, payoffs reduced by a
@@ -23,7 +26,6 @@
 
 namespace mpc {
 
-constexpr int kPlainBlock = 128;  // largest block
 template <int SMP>
 struct PlainSource {
   using type = Source<SMP>;
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(kPlainBlock, plain_min_blocks(FAM)) plain_kern
   const uint64_t first = (uint64_t)blockIdx.x * q.tile_units;
   const uint64_t last = min(first + (uint64_t)q.tile_units, q.n_units);
   double v[5] = {0, 0, 0, 0, 0};
-  for (uint64_t base = first; base < last; base += blockDim.x) {
+  for (uint64_t base = first; base < last; base += kPlainBlock) {
     // a thread past the end repeats the last unit and discards it (block- and
     // warp-synchronous sources need every thread)
     const bool valid = base + threadIdx.x < last;
@@ -95,36 +97,36 @@ __global__ void __launch_bounds__(kPlainBlock, plain_min_blocks(FAM)) plain_kern
 }
 
 template <int SMP>
-cudaError_t launch_plain_s(const DevReq& q, const DeviceTables& tabs, int block, cudaStream_t stream) {
+cudaError_t launch_plain_s(const DevReq& q, const DeviceTables& tabs, cudaStream_t stream) {
   SrcCtx ctx{tabs.sobol, tabs.jump, nullptr, nullptr, tabs.icdf_tail};
   const uint32_t grid = q.n_tiles;
   switch (q.family) {
     case FAM_GBM_STEP:
-      plain_kernel<FAM_GBM_STEP, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      plain_kernel<FAM_GBM_STEP, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     case FAM_GBM_TERMINAL:
-      plain_kernel<FAM_GBM_TERMINAL, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      plain_kernel<FAM_GBM_TERMINAL, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     case FAM_HESTON:
-      plain_kernel<FAM_HESTON, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      plain_kernel<FAM_HESTON, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     case FAM_BASKET:
-      plain_kernel<FAM_BASKET, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      plain_kernel<FAM_BASKET, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     case FAM_MLMC_LEVEL:
-      plain_kernel<FAM_MLMC_LEVEL, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      plain_kernel<FAM_MLMC_LEVEL, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     case FAM_GBM_BRIDGE:
       if constexpr (SMP != SMP_SOBOL) return cudaErrorInvalidValue;
-      else plain_kernel<FAM_GBM_BRIDGE, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      else plain_kernel<FAM_GBM_BRIDGE, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     case FAM_MERTON_STEP:  // the pseudorandom Merton is the stream replay (mpc_merton.cu)
       if constexpr (SMP == SMP_XORSHIFT) return cudaErrorInvalidValue;
-      else plain_kernel<FAM_MERTON_STEP, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      else plain_kernel<FAM_MERTON_STEP, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     case FAM_MERTON_TERMINAL:
       if constexpr (SMP == SMP_XORSHIFT) return cudaErrorInvalidValue;
-      else plain_kernel<FAM_MERTON_TERMINAL, SMP><<<grid, block, 0, stream>>>(q, ctx);
+      else plain_kernel<FAM_MERTON_TERMINAL, SMP><<<grid, kPlainBlock, 0, stream>>>(q, ctx);
       break;
     default:
       return cudaErrorInvalidValue;

@@ -2,6 +2,6 @@
 #include "mpc_plain.cuh"
 
 namespace mpc {
-template cudaError_t launch_plain_s<SMP_HALTON>(const DevReq&, const DeviceTables&, int, cudaStream_t);
-template cudaError_t launch_plain_s<SMP_LHS>(const DevReq&, const DeviceTables&, int, cudaStream_t);
+template cudaError_t launch_plain_s<SMP_HALTON>(const DevReq&, const DeviceTables&, cudaStream_t);
+template cudaError_t launch_plain_s<SMP_LHS>(const DevReq&, const DeviceTables&, cudaStream_t);
 }  // namespace mpc

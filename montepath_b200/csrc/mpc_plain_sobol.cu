@@ -2,11 +2,11 @@
 #include "mpc_plain.cuh"
 
 namespace mpc {
-extern template cudaError_t launch_plain_s<SMP_XORSHIFT>(const DevReq&, const DeviceTables&, int, cudaStream_t);
-extern template cudaError_t launch_plain_s<SMP_COUNTER>(const DevReq&, const DeviceTables&, int, cudaStream_t);
-extern template cudaError_t launch_plain_s<SMP_HALTON>(const DevReq&, const DeviceTables&, int, cudaStream_t);
-extern template cudaError_t launch_plain_s<SMP_LHS>(const DevReq&, const DeviceTables&, int, cudaStream_t);
-template cudaError_t launch_plain_s<SMP_SOBOL>(const DevReq&, const DeviceTables&, int, cudaStream_t);
+extern template cudaError_t launch_plain_s<SMP_XORSHIFT>(const DevReq&, const DeviceTables&, cudaStream_t);
+extern template cudaError_t launch_plain_s<SMP_COUNTER>(const DevReq&, const DeviceTables&, cudaStream_t);
+extern template cudaError_t launch_plain_s<SMP_HALTON>(const DevReq&, const DeviceTables&, cudaStream_t);
+extern template cudaError_t launch_plain_s<SMP_LHS>(const DevReq&, const DeviceTables&, cudaStream_t);
+template cudaError_t launch_plain_s<SMP_SOBOL>(const DevReq&, const DeviceTables&, cudaStream_t);
 
 // The lower tail of the FP64 inverse normal at the 23-bit midpoint uniforms.
 static __global__ void __launch_bounds__(256) icdf_tail_kernel(double* __restrict__ out) {
@@ -19,18 +19,18 @@ cudaError_t launch_icdf_tail(double* d_out, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_plain(const DevReq& q, int sampler, const DeviceTables& tabs, int block, cudaStream_t stream) {
+cudaError_t launch_plain(const DevReq& q, int sampler, const DeviceTables& tabs, cudaStream_t stream) {
   switch (sampler) {
     case SMP_XORSHIFT:
-      return launch_plain_s<SMP_XORSHIFT>(q, tabs, block, stream);
+      return launch_plain_s<SMP_XORSHIFT>(q, tabs, stream);
     case SMP_HALTON:
-      return launch_plain_s<SMP_HALTON>(q, tabs, block, stream);
+      return launch_plain_s<SMP_HALTON>(q, tabs, stream);
     case SMP_LHS:
-      return launch_plain_s<SMP_LHS>(q, tabs, block, stream);
+      return launch_plain_s<SMP_LHS>(q, tabs, stream);
     case SMP_SOBOL:
-      return launch_plain_s<SMP_SOBOL>(q, tabs, block, stream);
+      return launch_plain_s<SMP_SOBOL>(q, tabs, stream);
     case SMP_COUNTER:
-      return launch_plain_s<SMP_COUNTER>(q, tabs, block, stream);
+      return launch_plain_s<SMP_COUNTER>(q, tabs, stream);
     default:
       return cudaErrorInvalidValue;
   }

@@ -105,31 +105,31 @@ __global__ void __launch_bounds__(kPlainBlock, 4) plain_split_kernel(const __gri
   plain_finish(q, last - first, v, red, &s_last);
 }
 
-cudaError_t launch_plain_split(const DevReq& q, const DeviceTables& tabs, int block, uint32_t lanes, cudaStream_t stream) {
-  if (lanes < 2 || lanes > 32 || (lanes & (lanes - 1)) || q.tile_units * lanes != (uint32_t)block ||
+cudaError_t launch_plain_split(const DevReq& q, const DeviceTables& tabs, uint32_t lanes, cudaStream_t stream) {
+  if (lanes < 2 || lanes > 32 || (lanes & (lanes - 1)) || q.tile_units * lanes != kPlainBlock ||
       (q.n_steps / 2 + 1) / lanes + 1 > kPlainSplitNormals / 2)
     return cudaErrorInvalidValue;
   switch (q.workload) {
     case W_ASIAN:
-      plain_split_kernel<W_ASIAN><<<q.n_tiles, block, 0, stream>>>(q, tabs.jump, lanes);
+      plain_split_kernel<W_ASIAN><<<q.n_tiles, kPlainBlock, 0, stream>>>(q, tabs.jump, lanes);
       break;
     case W_DAO:
-      plain_split_kernel<W_DAO><<<q.n_tiles, block, 0, stream>>>(q, tabs.jump, lanes);
+      plain_split_kernel<W_DAO><<<q.n_tiles, kPlainBlock, 0, stream>>>(q, tabs.jump, lanes);
       break;
     case W_UAO:
-      plain_split_kernel<W_UAO><<<q.n_tiles, block, 0, stream>>>(q, tabs.jump, lanes);
+      plain_split_kernel<W_UAO><<<q.n_tiles, kPlainBlock, 0, stream>>>(q, tabs.jump, lanes);
       break;
     case W_LOOKBACK:
-      plain_split_kernel<W_LOOKBACK><<<q.n_tiles, block, 0, stream>>>(q, tabs.jump, lanes);
+      plain_split_kernel<W_LOOKBACK><<<q.n_tiles, kPlainBlock, 0, stream>>>(q, tabs.jump, lanes);
       break;
     default:
-      plain_split_kernel<W_EURO><<<q.n_tiles, block, 0, stream>>>(q, tabs.jump, lanes);
+      plain_split_kernel<W_EURO><<<q.n_tiles, kPlainBlock, 0, stream>>>(q, tabs.jump, lanes);
       break;
   }
   count_graph_launches(1);  // adds to the launch count
   return cudaGetLastError();
 }
 
-template cudaError_t launch_plain_s<SMP_XORSHIFT>(const DevReq&, const DeviceTables&, int, cudaStream_t);
-template cudaError_t launch_plain_s<SMP_COUNTER>(const DevReq&, const DeviceTables&, int, cudaStream_t);
+template cudaError_t launch_plain_s<SMP_XORSHIFT>(const DevReq&, const DeviceTables&, cudaStream_t);
+template cudaError_t launch_plain_s<SMP_COUNTER>(const DevReq&, const DeviceTables&, cudaStream_t);
 }  // namespace mpc

@@ -821,8 +821,11 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
   // The moments land in pinned memory, written by the kernels themselves.
   // When no group has more than kFusedInline requests, the descriptors travel
   // as kernel parameters and the call is the launches alone; else descriptors
-  // and tile lists are copied in first.  A 10,000-path terminal call: 51 us with
-  // two copies in, a counter fill and a copy out around the same kernel, 29 us.
+  // and tile lists are copied in first.  Four Asian requests of 1,000 x 16: 47 us
+  // with the copies, 31 inline; 50,000 x 64: 70 and 57.  The line is the size of the
+  // parameter block, which every launch copies whole: with room for 16 requests
+  // (20 KB instead of 5) one request takes 2 us more (10,000 x 64: 31.6 -> 33.6),
+  // while groups of 5 to 16 would take 10 to 15 us less.
   bool inlined = true;
   for (const Group& g : gl) inlined = inlined && g.members.size() <= kFusedInline;
   const size_t mom_bytes = n * MPC_MOMENTS * sizeof(double);
@@ -967,19 +970,20 @@ int run_fused(mpc_context* ctx, std::vector<Prepared*>& reqs, std::vector<mpc_re
 }
 
 // ------------------------------------------------------------ plain path ---
-// Threads per block of a plain launch: 128, or fewer while that leaves more of
-// the 148 SMs with a block (a block of 32 is one unit per lane of one warp).
-static uint32_t plain_block(uint64_t units) { return units >= 128 * 256 ? 128u : units >= 64 * 128 ? 64u : 32u; }
-
 // Threads per path of a plain launch: more than one for stepwise GBM on the
 // pseudorandom stream while the paths alone do not fill the FP64 pipes (16
-// warps on each of 148 SMs), as long as a thread keeps at least 8 normals (its
-// stream seek costs about as much as generating 4) and they fit its share.
-static uint32_t plain_lanes(const Prepared& p) {
+// warps on each SM), as long as a thread keeps at least 8 normals (its stream
+// seek costs about as much as generating 4) and they fit its share.  One lane
+// against the rule's lanes, 64 steps, device time: 5,000 paths 25.7 / 16.8 us (8
+// lanes), 20,000 28.8 / 22.5 (4), 40,000 32.5 / 32.3 (2); from 80,000 on one, since
+// two give 44 / 44 and four 52.  A share past kPlainSplitNormals falls back to one
+// lane: 20,000 x 126 takes 43 where 8 lanes take 35, 20,000 x 252 72 where 8 take 47.
+static uint32_t plain_lanes(int sm_count, const Prepared& p) {
   const DevReq& q = p.q;
   if (p.sampler != SMP_XORSHIFT || p.family != FAM_GBM_STEP) return 1;
+  const uint64_t enough = uint64_t(sm_count) * 512;
   uint32_t lanes = 1;
-  while (lanes < 32 && q.n_units * lanes < 148 * 512 && q.n_steps >= 16 * lanes) lanes *= 2;
+  while (lanes < 32 && q.n_units * lanes < enough && q.n_steps >= 16 * lanes) lanes *= 2;
   return (q.n_steps / 2 + 1) / lanes + 1 <= kPlainSplitNormals / 2 ? lanes : 1;
 }
 
@@ -995,13 +999,15 @@ static int run_plain(mpc_context* ctx, Prepared* p, mpc_result_t* out, double* p
                            q.cv ? units * sizeof(double) : 0, documented_reduction_bytes(units)},
                           {"plain_pay", "plain_part", "plain_done"})))
     return st;
-  const uint32_t lanes = plain_lanes(*p);
-  const uint32_t block = lanes > 1 ? 128u : plain_block(units);
-  // units per thread: 1, or up to 4 for units of a few samples, while the
-  // launch keeps several blocks per SM
+  const uint32_t lanes = plain_lanes(ctx->sm_count, *p);
+  // units per thread: 1, or up to 4 for units of a few samples (a block's tables
+  // and its reduction then serve more of them), while the launch keeps several
+  // blocks per SM.  1 / 2 / 4 units, Sobol: terminal (1 sample) 300,000 paths
+  // 21 / 17 / 15 us, 4,000,000 152 / 94 / 68; 4 steps 100,000 14.6 / 15.1 / 16.8,
+  // 4,000,000 192 / 135 / 109 (two by this rule); 8 steps 228 / 175 / 152 (one)
   uint32_t per_thread = 1;
-  while (per_thread < 4 && per_thread * q.normals_per_unit < 8 && units >= uint64_t(block) * per_thread * 2 * 1024) per_thread *= 2;
-  q.tile_units = lanes > 1 ? block / lanes : block * per_thread;
+  while (per_thread < 4 && per_thread * q.normals_per_unit < 8 && units >= uint64_t(kPlainBlock) * per_thread * 2 * 1024) per_thread *= 2;
+  q.tile_units = lanes > 1 ? kPlainBlock / lanes : kPlainBlock * per_thread;
   if (units > 0x7FFFFFFFull * q.tile_units) return fail(ctx, MPC_E_UNSUPPORTED, "too many tiles for one launch");
   q.n_tiles = uint32_t((units + q.tile_units - 1) / q.tile_units);
   void *d_pay = nullptr, *d_part, *d_done;
@@ -1019,8 +1025,8 @@ static int run_plain(mpc_context* ctx, Prepared* p, mpc_result_t* out, double* p
   q.per_unit = static_cast<double*>(d_pay);
   uint64_t launches_before = kernel_launch_count();
   MPC_CUDA(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
-  const cudaError_t e = lanes > 1 ? launch_plain_split(q, ctx->tabs, int(block), lanes, ctx->stream)
-                                  : launch_plain(q, p->sampler, ctx->tabs, int(block), ctx->stream);
+  const cudaError_t e = lanes > 1 ? launch_plain_split(q, ctx->tabs, lanes, ctx->stream)
+                                  : launch_plain(q, p->sampler, ctx->tabs, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "plain pricing kernel");
   MPC_CUDA(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
   MPC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
