@@ -315,8 +315,8 @@ __device__ __forceinline__ float counter_normal_fast(uint32_t seed, uint32_t pat
 // minimum instead of a test, and the angle needs neither (u = 0 and u = 1 have
 // the same cosine).  The kernels on counter-hash samples are bound by issue
 // (0.81 to 0.85 of the slots): 24 contracts of a book, single-asset part
-// (2.1e8 path-steps) 647 -> 375 us, 5-asset baskets (1.6e9 normals) 3,211 ->
-// 2,380 us (one normal at a time took 63 instructions there).
+// (2.1e8 path-steps) 647 -> 396 us, 5-asset baskets (1.6e9 normals) 3,211 ->
+// 2,434 us (one normal at a time took 63 instructions there).
 __device__ __forceinline__ float2 splat2(float x) { return make_float2(x, x); }
 template <bool HWCOS>
 __device__ __forceinline__ float2 counter_normal_pair(uint32_t a, uint32_t b) {

@@ -83,8 +83,8 @@ __device__ __forceinline__ void fused_unit_any(const DevReq& q, const SrcCtx& ct
 // Resident blocks per SM the register allocation must allow: the
 // family-switching instance is the widest; terminal paths on the counter hash
 // are one short chain that wants more warps (stepwise ones draw two normals at
-// a time and want the registers: 439 us with 40 of them, 375 us with 64, the
-// book's single-asset part).
+// a time and want the registers: 439 us with 40 of them, 375 us with 64 and 396
+// with __expf's range check, the book's single-asset part).
 constexpr int fused_min_blocks(int fam, int smp) {
   return fam < 0 ? 2 : (fam == FAM_GBM_TERMINAL && smp == SMP_COUNTER ? 6 : 4);
 }
@@ -795,8 +795,9 @@ __device__ __forceinline__ uint32_t next_scenario_tile(const DevReq& q, uint32_t
 // One request split into q.n_tiles tiles of q.tile_units units.  262,144
 // antithetic Asian paths x 64 steps on Sobol, 9 legs: 98 -> 85 us with the
 // normals by quads, the legs in the parameter bank and the rows summed by all
-// warps.  18 exponentials a normal: the MUFU pipe is at half its rate; three
-// (92 us) and four (86 us) blocks per SM are no faster than two.
+// warps (three and four blocks per SM 92 and 86 then); 100 us with __expf, whose
+// test for results below the normal range is 3 instructions on each of the 18
+// exponentials a normal and keeps such prices from being flushed to zero.
 template <int FAM, int SMP, int TECH>
 __global__ void __launch_bounds__(kFusedBlock, 2) scenario_kernel(const __grid_constant__ DevReq sq,
                                                                  const __grid_constant__ ScenarioLegs legs, SrcCtx ctx) {

@@ -475,6 +475,11 @@ constexpr bool kQuadSource<SobolQuad> = true;
 template <>
 constexpr bool kQuadSource<SobolPlain> = true;
 
+template <class S>
+constexpr bool kCounterSource = false;
+template <bool HWCOS>
+constexpr bool kCounterSource<CounterFastT<HWCOS>> = true;
+
 // Sources that give the normals of two consecutive dimensions at once (n2).
 template <class S>
 constexpr bool kPairSource = false;
@@ -1015,14 +1020,18 @@ __device__ __forceinline__ void sum_step_normals(Src& src, uint32_t n, Real zs[D
 // then D normals and D adds; correlating every step cost D (D + 1) / 2 + 2 D
 // more and held the Cholesky factor in registers through the whole path (64
 // registers a thread: 356 bytes spilled with D up to 8).  1.6e9 normals of
-// 5-asset baskets: 3,829 us, 3,211 us so, 2,380 us with the normals in pairs.
+// 5-asset baskets: 3,829 us, 3,211 us so, 2,434 us with the normals in pairs.
+// On the counter hash the final loop takes two assets a turn: whole, it spilled
+// 100 bytes inside the path (2,534 us); on the pseudorandom stream whole is up
+// to 9% faster.
 template <class Real, int D, class Src>
 __device__ __forceinline__ void unit_basket_d(const DevReq& q, Src& src, double& pay, double& ctl) {
   const uint32_t n = q.n_steps;
   Real zs[D];
   sum_step_normals<Real, D>(src, n, zs);
   Real b0 = 0, b1 = 0;
-#pragma unroll
+  constexpr int kTurn = kCounterSource<Src> ? 2 : D;  // assets a turn
+#pragma unroll kTurn
   for (int a = 0; a < D; ++a) {
     Real w = (Real)0;
 #pragma unroll
