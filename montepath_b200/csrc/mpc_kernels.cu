@@ -618,7 +618,7 @@ __device__ __forceinline__ void scen_gbm_step(const DevReq& q, Src& src, const f
       src.at_step(st, 4);
       src.quad_load(st);
       const float2 z01 = src.template take_n2<0, 1>(st), z23 = src.template take_n2<2, 3>(st);
-#pragma unroll 1
+#pragma unroll 2
       for (int k = 0; k < 4; ++k) advance(k == 0 ? z01.x : k == 1 ? z01.y : k == 2 ? z23.x : z23.y);
     }
   } else if constexpr (kPairSource<Src>) {
@@ -793,13 +793,15 @@ __device__ __forceinline__ uint32_t next_scenario_tile(const DevReq& q, uint32_t
 }
 
 // One request split into q.n_tiles tiles of q.tile_units units.  262,144
-// antithetic Asian paths x 64 steps on Sobol, 9 legs: 98 -> 85 us with the
-// normals by quads, the legs in the parameter bank and the rows summed by all
-// warps (three and four blocks per SM 92 and 86 then); 100 us with __expf, whose
-// test for results below the normal range is 3 instructions on each of the 18
-// exponentials a normal and keeps such prices from being flushed to zero.
+// antithetic Asian paths x 64 steps on Sobol, 9 legs: 98 -> 92 us with the
+// normals by quads (two steps a turn of the inner loop: one takes 100), the legs in
+// the parameter bank and the rows summed by all warps.  Bound by the 18
+// exponentials a normal and the chains around them (MUFU 45%, issue 65%).  Three
+// blocks per SM where a leg has one path (9 states in 80 registers: Asian x 64 on
+// the counter hash, 262,144 paths a report, 145 -> 122 us; 5,000 paths 52 and 52),
+// two for antithetic legs, whose 18 would spill (30,000 x 128 on Sobol 99 -> 105).
 template <int FAM, int SMP, int TECH>
-__global__ void __launch_bounds__(kFusedBlock, 2) scenario_kernel(const __grid_constant__ DevReq sq,
+__global__ void __launch_bounds__(kFusedBlock, TECH == kScenAnti ? 2 : 3) scenario_kernel(const __grid_constant__ DevReq sq,
                                                                  const __grid_constant__ ScenarioLegs legs, SrcCtx ctx) {
   constexpr int NM = TECH == kScenCv ? 5 : 2;  // moments per leg
   extern __shared__ __align__(16) uint32_t sobol_window[];
