@@ -270,7 +270,7 @@ typedef struct mpc_options {
   int32_t device;           /* CUDA device ordinal */
   int32_t deterministic;    /* reductions always run in fixed tile order, so results
                                are deterministic for 0 and 1 alike */
-  uint64_t hbm_budget_bytes; /* 0 = 64 GiB */
+  uint64_t hbm_budget_bytes; /* 0 = 64 GiB; the context's fixed FP64 tables (1.7 MB) are not charged to it */
   uint32_t default_block_size; /* 0 (autotuner), 128, 256 or 512: block size of fused
                                   launches when a request gives no hint and mpc_prepare
                                   has not tuned its kind (other values: MPC_E_UNSUPPORTED) */
@@ -422,7 +422,8 @@ int mpc_flush_l2(mpc_context_t* ctx);
 /* Device time (ms) of the last mpc_price / mpc_price_batch and the number of
  * kernels it launched. */
 int mpc_last_timing(const mpc_context_t* ctx, double* device_ms, uint64_t* kernel_launches);
-/* Host<->device bytes the last mpc_price / mpc_price_batch copied (no reference counterpart: diagnostics). */
+/* Host<->device bytes of the last mpc_price / mpc_price_batch (no reference counterpart: diagnostics): copies,
+ * descriptors that travelled as launch parameters, and results that kernels wrote to mapped host memory. */
 int mpc_last_transfer(const mpc_context_t* ctx, uint64_t* h2d_bytes, uint64_t* d2h_bytes);
 /* Measured FP32 FMA (TFLOP/s) and MUFU (Tops/s) throughput of the device, the
  * roofline denominators of the compute-bound fused kernels (no reference counterpart). */
